@@ -44,7 +44,7 @@ const void *single_kernel(int log2b, const Tuning &t, int variant) {
 }
 
 size_t batch_smem_bytes(int lut_smem_entries) {
-    return (size_t)lut_smem_entries * sizeof(float4) + (size_t)(lut_smem_entries + 1) * sizeof(int);
+    return (size_t)(lut_smem_entries + 2) * sizeof(float4) + (size_t)(lut_smem_entries + 1) * sizeof(int);
 }
 
 int max_batch_blocks_per_sm(int log2b, const Tuning &t, int lut_smem_entries, int variant) {

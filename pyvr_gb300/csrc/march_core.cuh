@@ -81,11 +81,6 @@ __device__ __forceinline__ float load_value(const uint2 *p) {
 }
 
 template <bool SMEM>
-__device__ __forceinline__ float4 lut_entry(const float4 *lut, int i) {
-    if (SMEM) return lut[i];
-    return __ldg(lut + i);
-}
-template <bool SMEM>
 __device__ __forceinline__ int prefix_entry(const int *p, int i) {
     if (SMEM) return p[i];
     return __ldg(p + i);
@@ -152,9 +147,18 @@ __device__ __forceinline__ void shade_sample(const MarchFrame &f, const Rec *__r
     const float lu = FAST ? fmaf(density, f.flut_size, -0.5f) : __fadd_rn(__fmul_rn(density, f.flut_size), -0.5f);
     const float lfl = floorf(lu);
     const float la = __fadd_rn(lu, -lfl);
-    const int i0 = lut_index(lfl, f.flut_max);
-    const int i1 = lut_index(__fadd_rn(lfl, 1.0f), f.flut_max);
-    const float4 A = lut_entry<SMEM_LUT>(lut, i0), B = lut_entry<SMEM_LUT>(lut, i1);
+    float4 A, B;
+    if (SMEM_LUT) {
+        // the staged table has an apron entry at either end (stage_lut), so one
+        // clamped index addresses both entries: -1 and 0 below the table (or
+        // for NaN), size - 1 and size above it
+        const float4 *e = lut + (int)fminf(fmaxf(lfl, -1.0f), f.flut_max);
+        A = e[0];
+        B = e[1];
+    } else {
+        A = __ldg(lut + lut_index(lfl, f.flut_max));
+        B = __ldg(lut + lut_index(__fadd_rn(lfl, 1.0f), f.flut_max));
+    }
     const float2 crg = lerp_tex2(lo2(A), lo2(B), la);
     const float2 cba = lerp_tex2(hi2(A), hi2(B), la);  // (blue, alpha_tf)
 
@@ -305,6 +309,25 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
     }
 }
 
+// The pixel of a lane in its warp's 8x4 block, in Z-order.  The L1 data pipe
+// serves a 16-byte gather in passes of 8 lanes and an 8-byte gather in passes
+// of 16, each taking longer the more 128-byte lines its lanes touch (it is
+// 80-88 % busy on the large frames): in Z-order a pass covers 4x2 or 4x4
+// pixels instead of 8x1 or 8x2.  Measured against row order: a 1024^2 frame
+// of 256^3 uint8 with float records 538 -> 497 us, a 512^2 frame of 384^3
+// with half records 84.7 -> 79.8 us.
+__device__ __forceinline__ int lane_x(int lane) { return (lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4); }
+__device__ __forceinline__ int lane_y(int lane) { return ((lane >> 1) & 1) | ((lane >> 2) & 2); }
+
+// Stages a job's LUT with an apron entry at either end (s_lut[0] = entry 0,
+// s_lut[1 + i] = entry i, s_lut[1 + size] = entry size - 1) and its prefix
+// counts in shared memory.
+__device__ __forceinline__ void stage_lut(float4 *s_lut, int *s_prefix, const JobDesc &job) {
+    const int size = job.f.lut_size;
+    for (int k = threadIdx.x; k < size + 2; k += kBatchThreads) s_lut[k] = job.lut[min(max(k - 1, 0), size - 1)];
+    for (int k = threadIdx.x; k <= size; k += kBatchThreads) s_prefix[k] = job.prefix[k];
+}
+
 template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
 __device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, const float4 *lut,
                                            const int *prefix, int lane) {
@@ -338,19 +361,20 @@ __device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, c
 // fast arithmetic (the launcher groups a batch's jobs by variant, so that
 // each kernel carries one march and stays within its register budget).  The
 // job table is the kernel's own parameter block (read through the constant
-// cache).  Dynamic shared memory (SMEM_LUT): p.lut_smem_entries float4 LUT
-// entries followed by as many + 1 prefix counts, at least every job's LUT.
+// cache).  Dynamic shared memory (SMEM_LUT): p.lut_smem_entries + 2 float4
+// entries (a LUT and its apron) and p.lut_smem_entries + 1 prefix counts;
+// p.lut_smem_entries is at least every job's LUT size.
 template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
 __global__ void __launch_bounds__(kBatchThreads, COMPACT ? 5 : 4)
 march_batch_kernel(const __grid_constant__ BatchParams p) {
     extern __shared__ float4 s_dyn[];
     float4 *s_lut = s_dyn;
-    int *s_prefix = reinterpret_cast<int *>(s_dyn + p.lut_smem_entries);
+    int *s_prefix = reinterpret_cast<int *>(s_dyn + p.lut_smem_entries + 2);
     __shared__ int s_tile, s_job_idx;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warps_x = p.tile_w >> 3;
-    const int sub_x = (warp % warps_x) * 8 + (lane & 7);
-    const int sub_y = (warp / warps_x) * 4 + (lane >> 3);
+    const int sub_x = (warp % warps_x) * 8 + lane_x(lane);
+    const int sub_y = (warp / warps_x) * 4 + lane_y(lane);
     int cur_job = -1;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -370,15 +394,14 @@ march_batch_kernel(const __grid_constant__ BatchParams p) {
         if (SMEM_LUT && j != cur_job) {
             // stage the job's LUT (the previous tile's readers passed the
             // barrier at the end of the last round)
-            for (int k = threadIdx.x; k < job.f.lut_size; k += kBatchThreads) s_lut[k] = job.lut[k];
-            for (int k = threadIdx.x; k <= job.f.lut_size; k += kBatchThreads) s_prefix[k] = job.prefix[k];
+            stage_lut(s_lut, s_prefix, job);
             __syncthreads();
             cur_job = j;
         }
         const int local = t - job.tile_base;
         const int px = (local % job.tiles_x) * p.tile_w + sub_x;
         const int py = (local / job.tiles_x) * p.tile_h + sub_y;
-        march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut : job.lut,
+        march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut + 1 : job.lut,
                                                                     SMEM_LUT ? s_prefix : job.prefix, lane);
         __syncthreads();  // s_tile / the staged LUT are rewritten next round
     }
@@ -396,19 +419,18 @@ __global__ void __launch_bounds__(kBatchThreads, COMPACT ? 6 : 5)
 march_single_kernel(const __grid_constant__ SingleParams p) {
     extern __shared__ float4 s_dyn[];
     float4 *s_lut = s_dyn;
-    int *s_prefix = reinterpret_cast<int *>(s_dyn + p.lut_smem_entries);
+    int *s_prefix = reinterpret_cast<int *>(s_dyn + p.lut_smem_entries + 2);
     const JobDesc &job = p.job;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warps_x = p.tile_w >> 3;
     if (SMEM_LUT) {
-        for (int k = threadIdx.x; k < job.f.lut_size; k += kBatchThreads) s_lut[k] = job.lut[k];
-        for (int k = threadIdx.x; k <= job.f.lut_size; k += kBatchThreads) s_prefix[k] = job.prefix[k];
+        stage_lut(s_lut, s_prefix, job);
         __syncthreads();
     }
     const int t = blockIdx.x;
-    const int px = (t % job.tiles_x) * p.tile_w + (warp % warps_x) * 8 + (lane & 7);
-    const int py = (t / job.tiles_x) * p.tile_h + (warp / warps_x) * 4 + (lane >> 3);
-    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut : job.lut,
+    const int px = (t % job.tiles_x) * p.tile_w + (warp % warps_x) * 8 + lane_x(lane);
+    const int py = (t / job.tiles_x) * p.tile_h + (warp / warps_x) * 4 + lane_y(lane);
+    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut + 1 : job.lut,
                                                                 SMEM_LUT ? s_prefix : job.prefix, lane);
 }
 
