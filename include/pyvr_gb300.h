@@ -361,11 +361,25 @@ int pvr_diff_forward(const pvr_diff_scene *scene, float *d_image, int *d_steps, 
 
 /* Backward of pvr_diff_forward: given dL/dimage, ADDS dL/dLUT (lut_size x 4)
  * into d_grad_lut and dL/dvoxel (D x H x W) into d_grad_volume (either may
- * be NULL: not computed).  Transmittance is rebuilt by a reverse march over
- * each ray; normals are held constant. */
+ * be NULL: not computed).  Each ray is marched a second time, beside the image;
+ * normals are held constant. */
 int pvr_diff_backward(const pvr_diff_scene *scene, const float *d_image, const int *d_steps,
                       const float *d_grad_image, float *d_grad_lut, float *d_grad_volume,
                       void *stream);
+
+/* The same two with device scratch of the caller's, in which the scene's texels
+ * are packed for the march (and voxel gradients gathered): several times
+ * faster.  pvr_diff_workspace gives the bytes that help (0: none do), and those
+ * of a backward with d_grad_volume.  The scratch holds
+ * nothing between calls, must be 16-byte aligned, and may be given back to
+ * its owner's stream-ordered pool once the call has returned.  With NULL, or
+ * fewer bytes, the calls are those above. */
+int pvr_diff_workspace(const pvr_diff_scene *scene, long long *bytes, long long *bytes_volume_gradient);
+int pvr_diff_forward_ws(const pvr_diff_scene *scene, float *d_image, int *d_steps, void *workspace,
+                        long long workspace_bytes, void *stream);
+int pvr_diff_backward_ws(const pvr_diff_scene *scene, const float *d_image, const int *d_steps,
+                         const float *d_grad_image, float *d_grad_lut, float *d_grad_volume, void *workspace,
+                         long long workspace_bytes, void *stream);
 
 /* ---- Serving runtime (no counterpart in the reference) -----------------
  * Continuous batching of render requests over resident volumes and LUTs on

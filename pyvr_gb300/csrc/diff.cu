@@ -4,35 +4,40 @@
 // Forward: the march of pyvr/shaders/volume.frag.glsl:70-122 with the
 // renderer's exact per-sample arithmetic (setup_ray, texel fractions,
 // z-then-y-then-x trilinear lerps, LUT lerp, pvr_expf opacity correction,
-// Lambert term, front-to-back compositing), reading the volume in its linear
-// (D, H, W) layout, so the float image equals the renderer's float image.
-// Per pixel it also keeps the number of loop iterations executed; nothing
-// is kept per sample.
+// Lambert term, front-to-back compositing), so the float image equals the
+// renderer's float image.  Per pixel it also keeps the number of loop
+// iterations executed; nothing is kept per sample.
 //
-// Backward: a second march over each ray in reverse order.  With T_i the
-// transmittance in front of sample i, c_i = light_i * rgb_i and
-// R_i the radiance behind sample i as seen from just after it,
-//   C = sum_i T_i alpha_i c_i,   A = 1 - prod_i (1 - alpha_i),
-//   dC/dc_i = T_i alpha_i,       dC/dalpha_i = T_i (c_i - R_i),
-//   dA/dalpha_i = T_i (1 - Ra_i),   Ra_i = 1 - prod_{j>i} (1 - alpha_j),
-// and walking from the last sample to the first, T_i = T_{i+1} / (1 - alpha_i)
-// starting from T_N = 1 - A, R_{i-1} = alpha_i c_i + (1 - alpha_i) R_i,
-// Ra_{i-1} = alpha_i + (1 - alpha_i) Ra_i.  The sample positions are those of
-// the forward march bit for bit: the position recurrence (repeated float
-// additions of one step) is replayed from the ray's start in segments of
-// kSeg iterations, each segment buffered and then walked backwards.  A
-// sample with alpha exactly 1 (transmittance not recoverable by division)
-// takes its T from a forward replay instead.
+// Backward: the same march a second time, front to back, with the forward's
+// own positions, samples and accumulators (bit for bit).  With T_i = 1 - acc.a
+// the transmittance in front of sample i, c_i = light_i * rgb_i and acc_i the
+// accumulated colour behind it, what lies beyond sample i is the image minus
+// acc_i, so
+//   dC/dc_i = T_i alpha_i,
+//   dC/dalpha_i = T_i c_i - (C - acc_i) / (1 - alpha_i),
+//   dA/dalpha_i = (1 - A) / (1 - alpha_i).
+// T_i is exact here (a walk from the last sample to the first has to rebuild
+// it by division from 1 - A), and all rays of a warp are at the same step,
+// so their gathers and table entries coincide as in the forward.  The last
+// sample of a ray has nothing beyond it: C - acc_i is exactly 0 there, and
+// dA/dalpha is T_i.
 //
 // Chain rule down to the leaves: alpha = 1 - exp(-a K) gives
 // dalpha/da = K exp(-a K); the LUT lerp rgba = lerp(lut[i0], lut[i1], f)
 // gives weights (1 - f, f) to the two entries and d rgba/d density =
 // (lut[i1] - lut[i0]) * lut_size; density = value_scale * trilinear(voxels)
 // gives each of the 8 corners its trilinear weight.  Normals (given, or
-// (density, 0, 0) without a normal volume) are held constant.  LUT gradients
-// are summed per warp over the lanes that address the same entries, then in
-// shared memory per block, and added to global memory once per block; voxel
-// gradients are added with global atomics.
+// (density, 0, 0) without a normal volume) are held constant.
+//
+// What bounds it, and the layout: a sample needs 8 texels of 1 (or, with
+// normals, 4) floats.  Gathered from the (D,H,W) and (D,H,W,3) arrays that
+// is 8 (32) loads, and the L1 data pipe is their limit (93 % busy).  With
+// a workspace (pvr_diff_workspace) each call first packs the volume into
+// 16-byte texels, which the march reads with 8 loads (value and normal of a
+// texel) or, without normals, 2 (the four (y, z) corners of a texel).
+// Measured on 128^3 with normals, 8 views of 512^2: forward 985 -> 515 us,
+// backward to the LUT 3250 -> 1020 us (with the front-to-back order), the packing 13 us of each; 72^3
+// without normals, 3 views of 251x197, backward to voxels and LUT 303 -> 110 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -47,28 +52,35 @@ namespace {
 constexpr int kDiffMaxViews = 32;   // views per launch (more are split)
 constexpr int kDiffThreads = 256;   // 16 x 16 pixel tile; warps cover 8 x 4 pixels
 constexpr int kDiffTile = 16;
-constexpr int kSeg = 16;            // reverse-march segment (iterations), buffered in shared memory
 constexpr int kDiffMaxLut = 2048;   // LUT entries (shared-memory gradient)
+// LUTs up to this many entries get a gradient table per warp (8 KB each),
+// larger ones one per block
+constexpr int kWarpTableLut = 512;
+
+// Where a sample's texels come from: the scene's arrays, or packed texels
+// with normals, or packed (y, z) quads of values.
+enum TexelSource { kLinear = 0, kPackedNormals = 1, kPackedQuads = 2 };
 
 struct DiffParams {
     const float *vol;       // (D, H, W) C order: texel (x, y, z) at (x * H + y) * D + z
     const float *nrm;       // 3 floats per texel, or null
+    const float4 *texels;   // packed texels (kPackedNormals, kPackedQuads)
     const float4 *lut;
     float4 *image;          // [view][y][x]
     int *steps;             // [view][y][x] loop iterations executed
     const float4 *gimage;   // dL/dimage
     float4 *glut;           // dL/dlut, accumulated; or null
     float *gvol;            // dL/dvoxel, accumulated; or null
+    float4 *gquads;         // dL/dvoxel by (y, z) quads (zeroed; added to gvol afterwards); or null
     int nviews, tiles_x, tiles_y;
     int ext[3];             // texels along world x, y, z (W, H, D)
     MarchFrame f[kDiffMaxViews];
 };
 
 struct Sample {
-    int x0, x1, y0, y1, z0, z1;
+    int k[3];        // lower texel, -1 .. ext - 1
     float fx, fy, fz;
-    float density;
-    int i0, i1;
+    int j0;          // LUT entry floor(lu) clamped to -1 .. size - 1
     float la;
     float4 A, B;
     float r, g, b;   // LUT colour
@@ -76,14 +88,6 @@ struct Sample {
     float alpha;     // 1 - e
     float light;     // ambient + diffuse * max(dot(n, L), 0)
 };
-
-__device__ __forceinline__ int texel(const DiffParams &p, int x, int y, int z) {
-    return (x * p.ext[1] + y) * p.ext[2] + z;
-}
-
-__device__ __forceinline__ int lut_idx(float fl, float lmax, int size) {
-    return !(fl >= 0.0f) ? 0 : (fl > lmax ? size - 1 : (int)fl);
-}
 
 // texture coordinate of a world position (frag:25-27, 88) and its validity
 __device__ __forceinline__ bool tex_coords(const MarchFrame &f, const float pos[3], float t[3]) {
@@ -100,64 +104,166 @@ __device__ __forceinline__ bool never_valid(const float t[3], const float d[3]) 
     return nv;
 }
 
+// Packed texels: texel clamp(i - 1) of each axis at index i in [0, ext + 1]
+// (kPackedNormals), so a footprint is never clamped; quads likewise along x,
+// and at (y, z) index (j, l) in [0, ext] the corners {(y, z), (y, z + 1),
+// (y + 1, z), (y + 1, z + 1)} of lower texel (j - 1, l - 1).
+__host__ __device__ inline long long packed_texels(const int ext[3], bool normals) {
+    return (long long)(ext[0] + 2) * (ext[1] + (normals ? 2 : 1)) * (ext[2] + (normals ? 2 : 1));
+}
+
+// Also clears the first nquads gradient quads (never more than the texels).
+template <int SOURCE>
+__global__ void pack_kernel(const float *__restrict__ vol, const float *__restrict__ nrm, int ex, int ey, int ez,
+                            float4 *__restrict__ out, float4 *__restrict__ gquads, int nquads) {
+    const int ny = ey + (SOURCE == kPackedNormals ? 2 : 1), nz = ez + (SOURCE == kPackedNormals ? 2 : 1);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int total = (ex + 2) * ny * nz;
+    if (i >= total) return;
+    if (i < nquads) gquads[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int z = i % nz, y = (i / nz) % ny, x = min(max(i / (nz * ny) - 1, 0), ex - 1);
+    const int y0 = min(max(y - 1, 0), ey - 1), z0 = min(max(z - 1, 0), ez - 1);
+    if (SOURCE == kPackedNormals) {
+        const int t = (x * ey + y0) * ez + z0;
+        out[i] = make_float4(vol[t], nrm[3 * t + 0], nrm[3 * t + 1], nrm[3 * t + 2]);
+    } else {
+        const int y1 = min(y, ey - 1), z1 = min(z, ez - 1);
+        const float *r0 = vol + (x * ey + y0) * ez, *r1 = vol + (x * ey + y1) * ez;
+        out[i] = make_float4(r0[z0], r0[z1], r1[z0], r1[z1]);
+    }
+}
+
+// dL/dvoxel from the quads: voxel (x, y, z) is the lower and the upper corner
+// of two quad indices per axis, and of one more at each clamped face.
+__global__ void unpack_grad_kernel(const float4 *__restrict__ quads, int ex, int ey, int ez, float *__restrict__ gvol) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ex * ey * ez) return;
+    const int z = i % ez, y = (i / ez) % ey, x = i / (ez * ey);
+    const int ny = ey + 1, nz = ez + 1;
+    float sum = 0.0f;
+    for (int qx = x == 0 ? 0 : x + 1; qx <= (x == ex - 1 ? ex + 1 : x + 1); ++qx) {
+        for (int qy = y; qy <= y + 1; ++qy)
+            for (int qz = z; qz <= z + 1; ++qz) {
+                const float4 q = __ldg(quads + (qx * ny + qy) * nz + qz);
+                // as lower corner: index c + 1, or 0 on the first texel; as
+                // upper corner: index c, or ext on the last
+                const bool yl = qy == y + 1 || y == 0, yu = qy == y || y == ey - 1;
+                const bool zl = qz == z + 1 || z == 0, zu = qz == z || z == ez - 1;
+                sum += (yl && zl ? q.x : 0.0f) + (yl && zu ? q.y : 0.0f) + (yu && zl ? q.z : 0.0f) +
+                       (yu && zu ? q.w : 0.0f);
+            }
+    }
+    gvol[i] += sum;
+}
+
+__device__ __forceinline__ int texel(const DiffParams &p, int x, int y, int z) {
+    return (x * p.ext[1] + y) * p.ext[2] + z;
+}
+
+// value (and normal) at a sample, from the scene's own arrays
 __device__ __forceinline__ float tri(const float *v, const DiffParams &p, const Sample &s, int stride, int c) {
-    const float v000 = __ldg(v + texel(p, s.x0, s.y0, s.z0) * stride + c);
-    const float v001 = __ldg(v + texel(p, s.x0, s.y0, s.z1) * stride + c);
-    const float v010 = __ldg(v + texel(p, s.x0, s.y1, s.z0) * stride + c);
-    const float v011 = __ldg(v + texel(p, s.x0, s.y1, s.z1) * stride + c);
-    const float v100 = __ldg(v + texel(p, s.x1, s.y0, s.z0) * stride + c);
-    const float v101 = __ldg(v + texel(p, s.x1, s.y0, s.z1) * stride + c);
-    const float v110 = __ldg(v + texel(p, s.x1, s.y1, s.z0) * stride + c);
-    const float v111 = __ldg(v + texel(p, s.x1, s.y1, s.z1) * stride + c);
+    int lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = max(s.k[a], 0);
+        hi[a] = min(s.k[a] + 1, p.ext[a] - 1);
+    }
+    const float v000 = __ldg(v + texel(p, lo[0], lo[1], lo[2]) * stride + c);
+    const float v001 = __ldg(v + texel(p, lo[0], lo[1], hi[2]) * stride + c);
+    const float v010 = __ldg(v + texel(p, lo[0], hi[1], lo[2]) * stride + c);
+    const float v011 = __ldg(v + texel(p, lo[0], hi[1], hi[2]) * stride + c);
+    const float v100 = __ldg(v + texel(p, hi[0], lo[1], lo[2]) * stride + c);
+    const float v101 = __ldg(v + texel(p, hi[0], lo[1], hi[2]) * stride + c);
+    const float v110 = __ldg(v + texel(p, hi[0], hi[1], lo[2]) * stride + c);
+    const float v111 = __ldg(v + texel(p, hi[0], hi[1], hi[2]) * stride + c);
     const float c0 = lerp_tex(lerp_tex(v000, v001, s.fz), lerp_tex(v010, v011, s.fz), s.fy);
     const float c1 = lerp_tex(lerp_tex(v100, v101, s.fz), lerp_tex(v110, v111, s.fz), s.fy);
     return lerp_tex(c0, c1, s.fx);
 }
 
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+
+// Stored value and normal at a sample; the lerps are the same per component
+// whatever the source.
+template <int SOURCE>
+__device__ __forceinline__ float fetch(const DiffParams &p, const MarchFrame &f, const Sample &s, float n[3]) {
+    if (SOURCE == kPackedNormals) {
+        const int sy = p.ext[2] + 2, sx = (p.ext[1] + 2) * sy;
+        const float4 *t = p.texels + ((s.k[0] + 1) * sx + (s.k[1] + 1) * sy + (s.k[2] + 1));
+        const float4 r000 = __ldg(t), r001 = __ldg(t + 1);
+        const float4 r010 = __ldg(t + sy), r011 = __ldg(t + sy + 1);
+        t += sx;
+        const float4 r100 = __ldg(t), r101 = __ldg(t + 1);
+        const float4 r110 = __ldg(t + sy), r111 = __ldg(t + sy + 1);
+        const float2 a = lerp_tex2(lerp_tex2(lerp_tex2(lo2(r000), lo2(r001), s.fz),
+                                             lerp_tex2(lo2(r010), lo2(r011), s.fz), s.fy),
+                                   lerp_tex2(lerp_tex2(lo2(r100), lo2(r101), s.fz),
+                                             lerp_tex2(lo2(r110), lo2(r111), s.fz), s.fy), s.fx);
+        const float2 b = lerp_tex2(lerp_tex2(lerp_tex2(hi2(r000), hi2(r001), s.fz),
+                                             lerp_tex2(hi2(r010), hi2(r011), s.fz), s.fy),
+                                   lerp_tex2(lerp_tex2(hi2(r100), hi2(r101), s.fz),
+                                             lerp_tex2(hi2(r110), hi2(r111), s.fz), s.fy), s.fx);
+        n[0] = a.y;
+        n[1] = b.x;
+        n[2] = b.y;
+        return __fmul_rn(a.x, f.value_scale);
+    }
+    float density;
+    if (SOURCE == kPackedQuads) {
+        const int sy = p.ext[2] + 1, sx = (p.ext[1] + 1) * sy;
+        const float4 *t = p.texels + ((s.k[0] + 1) * sx + (s.k[1] + 1) * sy + (s.k[2] + 1));
+        const float4 q0 = __ldg(t), q1 = __ldg(t + sx);
+        const float2 z0 = lerp_tex2(make_float2(q0.x, q0.z), make_float2(q0.y, q0.w), s.fz);
+        const float2 z1 = lerp_tex2(make_float2(q1.x, q1.z), make_float2(q1.y, q1.w), s.fz);
+        const float2 y = lerp_tex2(make_float2(z0.x, z1.x), make_float2(z0.y, z1.y), s.fy);
+        density = __fmul_rn(lerp_tex(y.x, y.y, s.fx), f.value_scale);
+    } else {
+        density = __fmul_rn(tri(p.vol, p, s, 1, 0), f.value_scale);
+        if (p.nrm) {
+            n[0] = tri(p.nrm, p, s, 3, 0);
+            n[1] = tri(p.nrm, p, s, 3, 1);
+            n[2] = tri(p.nrm, p, s, 3, 2);
+            return density;
+        }
+    }
+    // the reference's unbound normal sampler reads the volume
+    n[0] = density;
+    n[1] = 0.0f;
+    n[2] = 0.0f;
+    return density;
+}
+
 // Everything one in-box sample computes (frag:93-110), with the renderer's
-// rounding.  full: also the colour and the light term.
+// rounding.  lut: the table in shared memory with an apron entry at either
+// end (lut[-1] = lut[0], lut[size] = lut[size - 1]).
+template <int SOURCE>
 __device__ __forceinline__ void eval_sample(const DiffParams &p, const MarchFrame &f, const float t[3],
-                                           bool full, Sample &s) {
-    int lo[3], hi[3];
+                                           const float4 *lut, Sample &s) {
     float fr[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float u = __fadd_rn(__fmul_rn(t[a], f.fext[a]), -0.5f);
         const float fl = floorf(u);
         fr[a] = __fadd_rn(u, -fl);
-        const int k = (int)fl;  // -1 .. ext-1
-        lo[a] = max(k, 0);
-        hi[a] = min(k + 1, p.ext[a] - 1);
+        s.k[a] = (int)fl;  // -1 .. ext-1
     }
-    s.x0 = lo[0]; s.x1 = hi[0]; s.y0 = lo[1]; s.y1 = hi[1]; s.z0 = lo[2]; s.z1 = hi[2];
     s.fx = fr[0]; s.fy = fr[1]; s.fz = fr[2];
-    s.density = __fmul_rn(tri(p.vol, p, s, 1, 0), f.value_scale);
+    float n[3];
+    const float density = fetch<SOURCE>(p, f, s, n);
     // texture(transfer_function_lut, vec2(density, 0.5)) (frag:96)
-    const float lu = __fadd_rn(__fmul_rn(s.density, f.flut_size), -0.5f);
+    const float lu = __fadd_rn(__fmul_rn(density, f.flut_size), -0.5f);
     const float lfl = floorf(lu);
     s.la = __fadd_rn(lu, -lfl);
-    const float lmax = (float)(f.lut_size - 1);
-    s.i0 = lut_idx(lfl, lmax, f.lut_size);
-    s.i1 = lut_idx(__fadd_rn(lfl, 1.0f), lmax, f.lut_size);
-    s.A = __ldg(p.lut + s.i0);
-    s.B = __ldg(p.lut + s.i1);
-    const float a_tf = lerp_tex(s.A.w, s.B.w, s.la);
-    s.e = pvr_expf(-__fmul_rn(a_tf, f.alpha_k));
+    s.j0 = (int)fminf(fmaxf(lfl, -1.0f), f.flut_max);  // NaN: -1
+    s.A = lut[s.j0];
+    s.B = lut[s.j0 + 1];
+    const float2 rg = lerp_tex2(lo2(s.A), lo2(s.B), s.la), ba = lerp_tex2(hi2(s.A), hi2(s.B), s.la);
+    s.r = rg.x;
+    s.g = rg.y;
+    s.b = ba.x;
+    s.e = pvr_expf(-__fmul_rn(ba.y, f.alpha_k));
     s.alpha = __fadd_rn(1.0f, -s.e);
-    if (!full) return;
-    s.r = lerp_tex(s.A.x, s.B.x, s.la);
-    s.g = lerp_tex(s.A.y, s.B.y, s.la);
-    s.b = lerp_tex(s.A.z, s.B.z, s.la);
-    float n[3];
-    if (p.nrm) {
-        n[0] = tri(p.nrm, p, s, 3, 0);
-        n[1] = tri(p.nrm, p, s, 3, 1);
-        n[2] = tri(p.nrm, p, s, 3, 2);
-    } else {  // the reference's unbound normal sampler reads the volume
-        n[0] = s.density;
-        n[1] = 0.0f;
-        n[2] = 0.0f;
-    }
     const float n2 = __fadd_rn(__fadd_rn(__fmul_rn(n[0], n[0]), __fmul_rn(n[1], n[1])), __fmul_rn(n[2], n[2]));
     float di = 0.0f;
     if (n2 > 0.0f) {
@@ -170,38 +276,56 @@ __device__ __forceinline__ void eval_sample(const DiffParams &p, const MarchFram
     s.light = __fadd_rn(f.ambient, __fmul_rn(f.diffuse, di));
 }
 
-__device__ __forceinline__ void pixel_of(int tile_in_view, int tiles_x, int &px, int &py) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    px = (tile_in_view % tiles_x) * kDiffTile + (warp & 1) * 8 + (lane & 7);
-    py = (tile_in_view / tiles_x) * kDiffTile + (warp >> 1) * 4 + (lane >> 3);
+// acc.c += (1 - acc.a) * (c * light * alpha); acc.a += (1 - acc.a) * alpha
+__device__ __forceinline__ void composite(const Sample &s, float4 &acc) {
+    const float tr = __fadd_rn(1.0f, -acc.w);
+    acc.x = __fadd_rn(acc.x, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.r, s.light), s.alpha)));
+    acc.y = __fadd_rn(acc.y, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.g, s.light), s.alpha)));
+    acc.z = __fadd_rn(acc.z, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.b, s.light), s.alpha)));
+    acc.w = __fadd_rn(acc.w, __fmul_rn(tr, s.alpha));
 }
 
+// Lanes in Z-order inside the warp's 8x4 pixels, as in the renderer's march:
+// the 8 lanes of one pass of a 16-byte gather cover 4x2 pixels.
+__device__ __forceinline__ void pixel_of(int tile_in_view, int tiles_x, int &px, int &py) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    px = (tile_in_view % tiles_x) * kDiffTile + (warp & 1) * 8 +
+         ((lane & 1) | ((lane >> 1) & 2) | ((lane >> 2) & 4));
+    py = (tile_in_view / tiles_x) * kDiffTile + (warp >> 1) * 4 + (((lane >> 1) & 1) | ((lane >> 2) & 2));
+}
+
+__device__ __forceinline__ const float4 *stage_diff_lut(const DiffParams &p, float4 *s_lut) {
+    const int size = p.f[0].lut_size;
+    for (int k = threadIdx.x; k < size + 2; k += kDiffThreads) s_lut[k] = __ldg(p.lut + min(max(k - 1, 0), size - 1));
+    return s_lut + 1;
+}
+
+// Dynamic shared memory: the LUT and its apron (lut_size + 2 entries).
+template <int SOURCE>
 __global__ void __launch_bounds__(kDiffThreads)
 diff_forward_kernel(const __grid_constant__ DiffParams p) {
+    extern __shared__ float4 s_dyn[];
+    const float4 *lut = stage_diff_lut(p, s_dyn);
+    __syncthreads();
     const int per_view = p.tiles_x * p.tiles_y;
     const int view = blockIdx.x / per_view;
     const MarchFrame &f = p.f[view];
     int px, py;
     pixel_of(blockIdx.x % per_view, p.tiles_x, px, py);
     if (px >= f.width || py >= f.height) return;
-    float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, acc_a = 0.0f;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     int i = 0;
     float pos[3], d[3];
     if (setup_ray(f, px, py, pos, d)) {
         bool entered = false;
         for (;; ++i) {
-            if (!(i < f.max_steps && acc_a < 0.99f)) break;
+            if (!(i < f.max_steps && acc.w < 0.99f)) break;
             float t[3];
             if (tex_coords(f, pos, t)) {
                 entered = true;
                 Sample s;
-                eval_sample(p, f, t, true, s);
-                // acc.c += (1 - acc.a) * (c * light * alpha); acc.a += (1 - acc.a) * alpha
-                const float tr = __fadd_rn(1.0f, -acc_a);
-                acc_r = __fadd_rn(acc_r, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.r, s.light), s.alpha)));
-                acc_g = __fadd_rn(acc_g, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.g, s.light), s.alpha)));
-                acc_b = __fadd_rn(acc_b, __fmul_rn(tr, __fmul_rn(__fmul_rn(s.b, s.light), s.alpha)));
-                acc_a = __fadd_rn(acc_a, __fmul_rn(tr, s.alpha));
+                eval_sample<SOURCE>(p, f, t, lut, s);
+                composite(s, acc);
             } else if (entered || never_valid(t, d)) {
                 break;
             }
@@ -210,31 +334,27 @@ diff_forward_kernel(const __grid_constant__ DiffParams p) {
         }
     }
     const long long idx = ((long long)view * f.height + py) * f.width + px;
-    p.image[idx] = make_float4(acc_r, acc_g, acc_b, acc_a);
+    p.image[idx] = acc;
     p.steps[idx] = i;
-}
-
-// 1 - acc.a just before iteration `upto` of the forward march
-__device__ float replay_transmittance(const DiffParams &p, const MarchFrame &f, const float pos0[3],
-                                      const float d[3], int upto) {
-    float pos[3] = {pos0[0], pos0[1], pos0[2]};
-    float acc_a = 0.0f;
-    for (int i = 0; i < upto; ++i) {
-        float t[3];
-        if (tex_coords(f, pos, t)) {
-            Sample s;
-            eval_sample(p, f, t, false, s);
-            acc_a = __fadd_rn(acc_a, __fmul_rn(__fadd_rn(1.0f, -acc_a), s.alpha));
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) pos[a] = __fadd_rn(pos[a], d[a]);
-    }
-    return __fadd_rn(1.0f, -acc_a);
 }
 
 __device__ __forceinline__ void add_voxel_grad(const DiffParams &p, const Sample &s, float gd) {
     const float wx[2] = {1.0f - s.fx, s.fx}, wy[2] = {1.0f - s.fy, s.fy}, wz[2] = {1.0f - s.fz, s.fz};
-    const int xs[2] = {s.x0, s.x1}, ys[2] = {s.y0, s.y1}, zs[2] = {s.z0, s.z1};
+    if (p.gquads) {
+        // one 16-byte reduction per x corner
+        const int sy = p.ext[2] + 1, sx = (p.ext[1] + 1) * sy;
+        float4 *q = p.gquads + ((s.k[0] + 1) * sx + (s.k[1] + 1) * sy + (s.k[2] + 1));
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const float w0 = gd * wx[a] * wy[0], w1 = gd * wx[a] * wy[1];
+            atomicAdd(q + a * sx, make_float4(w0 * wz[0], w0 * wz[1], w1 * wz[0], w1 * wz[1]));
+        }
+        return;
+    }
+    int xs[2], ys[2], zs[2];
+    xs[0] = max(s.k[0], 0); xs[1] = min(s.k[0] + 1, p.ext[0] - 1);
+    ys[0] = max(s.k[1], 0); ys[1] = min(s.k[1] + 1, p.ext[1] - 1);
+    zs[0] = max(s.k[2], 0); zs[1] = min(s.k[2] + 1, p.ext[2] - 1);
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -248,25 +368,25 @@ __device__ __forceinline__ void add_voxel_grad(const DiffParams &p, const Sample
         }
 }
 
-// Sums v[0..7] over each group of lanes in `peers` (the lanes of `active`
+// Sums v[0..7] over each group of lanes in `peers` (the lanes of the warp
 // with the same key, from __match_any_sync) by a tree over the group's
 // ranks; returns true on the group's lowest lane, which then holds the sums.
-// Every lane of `active` must call it.
-__device__ __forceinline__ bool reduce_peers(unsigned active, unsigned peers, float v[8]) {
+// All lanes of the warp call it.
+__device__ __forceinline__ bool reduce_peers(unsigned peers, float v[8]) {
     const int lane = threadIdx.x & 31;
     int rank = __popc(peers & ((1u << lane) - 1u));
     unsigned above = lane == 31 ? 0u : peers & (0xffffffffu << (lane + 1));
     bool member = true;  // still holds a partial sum of its group
-    while (__any_sync(active, member && above != 0u)) {
+    while (__any_sync(0xffffffffu, member && above != 0u)) {
         const int next = (member && above) ? __ffs(above) - 1 : lane;
         const bool take = member && above != 0u && !(rank & 1);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const float t = __shfl_sync(active, v[c], next);
+            const float t = __shfl_sync(0xffffffffu, v[c], next);
             if (take) v[c] += t;
         }
         // the odd ranks have handed their sums down and leave
-        const unsigned leaving = __ballot_sync(active, member && (rank & 1));
+        const unsigned leaving = __ballot_sync(0xffffffffu, member && (rank & 1));
         if (member && (rank & 1)) member = false;
         above &= ~leaving;
         rank >>= 1;
@@ -274,93 +394,107 @@ __device__ __forceinline__ bool reduce_peers(unsigned active, unsigned peers, fl
     return member;
 }
 
-__device__ void backward_ray(const DiffParams &p, const MarchFrame &f, int px, int py, long long idx,
-                             float *s_glut, float *s_seg) {
-    const int nsteps = p.steps[idx];
-    if (nsteps <= 0) return;
-    const float4 g = p.gimage[idx];
-    if (g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f) return;
-    float pos0[3], d[3];
-    if (!setup_ray(f, px, py, pos0, d)) return;
-    const float4 out = p.image[idx];
-    float T = __fadd_rn(1.0f, -out.w);
-    float Rr = 0.0f, Rg = 0.0f, Rb = 0.0f, Ra = 0.0f;
-    // this thread's kSeg x 3 positions, strided by the block size (no bank
-    // conflicts between the lanes of a warp)
-    float *seg = s_seg + threadIdx.x;
-    int end = nsteps;
-    while (end > 0) {
-        const int start = max(0, end - kSeg);
-        float q[3] = {pos0[0], pos0[1], pos0[2]};
-        for (int k = 0; k < start; ++k)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) q[a] = __fadd_rn(q[a], d[a]);
-        for (int k = start; k < end; ++k) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                seg[((k - start) * 3 + a) * kDiffThreads] = q[a];
-                q[a] = __fadd_rn(q[a], d[a]);
-            }
-        }
-        for (int k = end - 1; k >= start; --k) {
-            float t[3];
-            const float bpos[3] = {seg[((k - start) * 3 + 0) * kDiffThreads], seg[((k - start) * 3 + 1) * kDiffThreads],
-                                   seg[((k - start) * 3 + 2) * kDiffThreads]};
-            if (!tex_coords(f, bpos, t)) continue;
+// A warp's rays of one tile.  table: the warp's own LUT gradient (WARP_TABLE:
+// entry j of the LUT at table[j + 1], its apron below and above, written
+// without atomics: the lanes that write hold different entries), or the
+// block's (channel-major floats, added to atomically); null without a LUT
+// gradient.  The whole warp runs every step.
+template <int SOURCE, bool WARP_TABLE>
+__device__ __forceinline__ void backward_rays(const DiffParams &p, const MarchFrame &f, int px, int py,
+                                              long long idx, const float4 *lut, float4 *table) {
+    int nsteps = px < f.width && py < f.height ? p.steps[idx] : 0;
+    float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f), out = g;
+    float pos[3] = {}, d[3] = {};
+    if (nsteps > 0) {
+        g = p.gimage[idx];
+        out = p.image[idx];
+        if ((g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f) || !setup_ray(f, px, py, pos, d)) nsteps = 0;
+    }
+    const float t_end = __fadd_rn(1.0f, -out.w);
+    const int most = __reduce_max_sync(0xffffffffu, nsteps);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = 0; i < most; ++i) {
+        float t[3];
+        const bool sampled = tex_coords(f, pos, t) && i < nsteps;
+        unsigned key = 0xffff0000u | threadIdx.x;  // no peers
+        float v[8];
+        if (sampled) {
             Sample s;
-            eval_sample(p, f, t, true, s);
-            const float om = 1.0f - s.alpha;
-            const float Ti = om > 0.0f ? T / om : replay_transmittance(p, f, pos0, d, k);
+            eval_sample<SOURCE>(p, f, t, lut, s);
+            const float T = __fadd_rn(1.0f, -acc.w);
+            composite(s, acc);
+            const float om = 1.0f - s.alpha, inv = om > 0.0f ? 1.0f / om : 0.0f;
             const float cr = s.light * s.r, cg = s.light * s.g, cb = s.light * s.b;
-            const float dalpha = Ti * (g.x * (cr - Rr) + g.y * (cg - Rg) + g.z * (cb - Rb) + g.w * (1.0f - Ra));
-            const float kc = Ti * s.light * s.alpha;
+            // T * (c - radiance behind) and T * (1 - alpha behind)
+            const float br = (out.x - acc.x) * inv, bg = (out.y - acc.y) * inv, bb = (out.z - acc.z) * inv;
+            const float ta = i == nsteps - 1 || !(om > 0.0f) ? T : t_end * inv;
+            const float dalpha = g.x * (T * cr - br) + g.y * (T * cg - bg) + g.z * (T * cb - bb) + g.w * ta;
+            const float kc = T * s.light * s.alpha;
             const float dr = g.x * kc, dg = g.y * kc, db = g.z * kc;
             const float da = dalpha * f.alpha_k * s.e;
-            if (s_glut) {
-                // neighbouring rays of a warp mostly address the same LUT
-                // entries: the lanes with the same pair of entries sum their
-                // contributions first, and one lane per pair adds them
-                const float w1 = s.la, w0 = 1.0f - s.la;
-                float v[8] = {w0 * dr, w0 * dg, w0 * db, w0 * da, w1 * dr, w1 * dg, w1 * db, w1 * da};
-                const unsigned active = __activemask();
-                const unsigned peers = __match_any_sync(active, ((unsigned)s.i0 << 16) | (unsigned)s.i1);
-                if (reduce_peers(active, peers, v)) {
-                    const int n = f.lut_size;  // channel-major: s_glut[c * n + entry]
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (v[c] != 0.0f) atomicAdd(s_glut + c * n + s.i0, v[c]);
-                        if (v[4 + c] != 0.0f) atomicAdd(s_glut + c * n + s.i1, v[4 + c]);
-                    }
-                }
-            }
+            const float w1 = s.la, w0 = 1.0f - s.la;
+            v[0] = w0 * dr; v[1] = w0 * dg; v[2] = w0 * db; v[3] = w0 * da;
+            v[4] = w1 * dr; v[5] = w1 * dg; v[6] = w1 * db; v[7] = w1 * da;
+            key = (unsigned)(s.j0 + 1);
             if (p.gvol) {
                 const float gd = (dr * (s.B.x - s.A.x) + dg * (s.B.y - s.A.y) + db * (s.B.z - s.A.z) +
                                   da * (s.B.w - s.A.w)) * f.flut_size * f.value_scale;
                 if (gd != 0.0f) add_voxel_grad(p, s, gd);
             }
-            Rr = cr * s.alpha + om * Rr;
-            Rg = cg * s.alpha + om * Rg;
-            Rb = cb * s.alpha + om * Rb;
-            Ra = s.alpha + om * Ra;
-            T = Ti;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = 0.0f;
         }
-        end = start;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) pos[a] = __fadd_rn(pos[a], d[a]);
+        if (table) {
+            // neighbouring rays of a warp mostly address the same entries: the
+            // lanes with the same entries sum their contributions first, and
+            // one lane per entry adds them
+            const unsigned peers = __match_any_sync(0xffffffffu, key);
+            const bool leader = reduce_peers(peers, v) && key < 0xffff0000u;
+            if (WARP_TABLE) {
+                if (leader) {
+                    float4 e = table[key];
+                    e.x += v[0]; e.y += v[1]; e.z += v[2]; e.w += v[3];
+                    table[key] = e;
+                }
+                __syncwarp();
+                if (leader) {
+                    float4 e = table[key + 1];
+                    e.x += v[4]; e.y += v[5]; e.z += v[6]; e.w += v[7];
+                    table[key + 1] = e;
+                }
+                __syncwarp();
+            } else if (leader) {
+                float *s_glut = reinterpret_cast<float *>(table);
+                const int n = f.lut_size, i0 = max((int)key - 1, 0), i1 = min((int)key, n - 1);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (v[c] != 0.0f) atomicAdd(s_glut + c * n + i0, v[c]);
+                    if (v[4 + c] != 0.0f) atomicAdd(s_glut + c * n + i1, v[4 + c]);
+                }
+            }
+        }
     }
 }
 
-// Dynamic shared memory: the reverse march's position segments (kSeg x 3
-// floats per thread), then the block's LUT gradient (4 x lut_size floats,
-// channel-major) when the LUT gradient is wanted.
+// Persistent blocks over the tiles.  Dynamic shared memory: the LUT and its
+// apron, then (p.glut) the gradient tables: one of lut_size + 2 entries per
+// warp, or one channel-major table per block.
+template <int SOURCE, bool WARP_TABLE>
 __global__ void __launch_bounds__(kDiffThreads)
 diff_backward_kernel(const __grid_constant__ DiffParams p) {
-    extern __shared__ float s_dyn[];
-    float *s_seg = s_dyn;
-    float *s_glut = s_dyn + kSeg * 3 * kDiffThreads;
-    const int lut_floats = 4 * p.f[0].lut_size;
-    if (p.glut) {
-        for (int k = threadIdx.x; k < lut_floats; k += kDiffThreads) s_glut[k] = 0.0f;
-        __syncthreads();
-    }
+    extern __shared__ float4 s_dyn[];
+    constexpr int kWarps = kDiffThreads / 32;
+    const int size = p.f[0].lut_size, rows = size + 2;
+    const float4 *lut = stage_diff_lut(p, s_dyn);
+    float4 *tables = s_dyn + rows;
+    if (p.glut)
+        for (int k = threadIdx.x; k < (WARP_TABLE ? kWarps * rows : size); k += kDiffThreads)
+            tables[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncthreads();
+    float4 *table = !p.glut ? nullptr : WARP_TABLE ? tables + (threadIdx.x >> 5) * rows : tables;
     const int per_view = p.tiles_x * p.tiles_y;
     const int total = per_view * p.nviews;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
@@ -368,16 +502,26 @@ diff_backward_kernel(const __grid_constant__ DiffParams p) {
         const MarchFrame &f = p.f[view];
         int px, py;
         pixel_of(tile % per_view, p.tiles_x, px, py);
-        if (px < f.width && py < f.height)
-            backward_ray(p, f, px, py, ((long long)view * f.height + py) * f.width + px,
-                         p.glut ? s_glut : nullptr, s_seg);
+        backward_rays<SOURCE, WARP_TABLE>(p, f, px, py, ((long long)view * f.height + py) * f.width + px, lut, table);
     }
-    if (p.glut) {
-        __syncthreads();
-        float *g = reinterpret_cast<float *>(p.glut);  // (lut_size, 4), entry-major
-        const int n = p.f[0].lut_size;
-        for (int k = threadIdx.x; k < lut_floats; k += kDiffThreads)
-            if (s_glut[k] != 0.0f) atomicAdd(g + 4 * (k % n) + k / n, s_glut[k]);
+    if (!p.glut) return;
+    __syncthreads();
+    float *g = reinterpret_cast<float *>(p.glut);  // (size, 4), entry-major
+    const float *flat = reinterpret_cast<const float *>(tables);
+    for (int k = threadIdx.x; k < 4 * size; k += kDiffThreads) {
+        float sum = 0.0f;
+        if (WARP_TABLE) {
+            const int e = k >> 2, c = k & 3;
+            for (int w = 0; w < kWarps; ++w) {
+                const float *t = flat + 4 * w * rows + c;
+                sum += t[4 * (e + 1)];
+                if (e == 0) sum += t[0];
+                if (e == size - 1) sum += t[4 * (size + 1)];
+            }
+        } else {
+            sum = flat[(k & 3) * size + (k >> 2)];
+        }
+        if (sum != 0.0f) atomicAdd(g + k, sum);
     }
 }
 
@@ -422,6 +566,7 @@ int build_params(const pvr_diff_scene *s, int v0, int nv, DiffParams &p) {
         f.value_scale = s->value_scale;
         f.lut_size = s->lut_size;
         f.flut_size = (float)s->lut_size;
+        f.flut_max = (float)(s->lut_size - 1);
     }
     return PVR_OK;
 }
@@ -444,26 +589,156 @@ int check_scene(const pvr_diff_scene *s) {
     return PVR_OK;
 }
 
+// Packing pays while a texel is read often enough: packing moves 44 bytes per
+// texel (about 7 ps), the march saves about 0.2 ns per ray and more.
+constexpr int kPackTexelsPerPixel = 16;
+
+long long packed_bytes(const pvr_diff_scene *s, bool normals) {
+    const int ext[3] = {s->w, s->h, s->d};
+    const long long n = packed_texels(ext, normals);
+    const long long pixels = (long long)s->width * s->height * s->n_views;
+    if (n > (1LL << 30) || (long long)s->d * s->h * s->w > kPackTexelsPerPixel * pixels) return 0;
+    return n * (long long)sizeof(float4);
+}
+
+int check_workspace(void *ws, long long bytes) {
+    if (ws && (reinterpret_cast<uintptr_t>(ws) & 15)) return fail(PVR_ERR_VALUE, "workspace must be 16-byte aligned");
+    if (bytes < 0) return fail(PVR_ERR_VALUE, "workspace bytes must be >= 0");
+    return PVR_OK;
+}
+
+// Packs the scene's texels into the workspace where that pays and fits, and
+// (volume_gradient) clears the gradient quads behind them: where the march
+// then reads and adds.
+struct Packed {
+    int source = kLinear;
+    const float4 *texels = nullptr;
+    float4 *gquads = nullptr;
+};
+cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, void *ws, long long bytes, cudaStream_t st,
+                       Packed &out) {
+    const long long need = packed_bytes(s, s->normals != nullptr), more = packed_bytes(s, false);
+    if (!ws || need == 0 || bytes < need) return cudaSuccess;
+    float4 *texels = static_cast<float4 *>(ws);
+    const int total = (int)(need / (long long)sizeof(float4)), blocks = (total + 255) / 256;
+    out.source = s->normals ? kPackedNormals : kPackedQuads;
+    out.texels = texels;
+    int nquads = 0;
+    if (volume_gradient && bytes >= need + more) {
+        out.gquads = texels + total;
+        nquads = (int)(more / (long long)sizeof(float4));
+    }
+    if (s->normals)
+        pack_kernel<kPackedNormals><<<blocks, 256, 0, st>>>(s->volume, s->normals, s->w, s->h, s->d, texels,
+                                                            out.gquads, nquads);
+    else
+        pack_kernel<kPackedQuads><<<blocks, 256, 0, st>>>(s->volume, nullptr, s->w, s->h, s->d, texels, out.gquads,
+                                                          nquads);
+    return cudaGetLastError();
+}
+
+const void *forward_kernel(int source) {
+    return source == kPackedNormals ? (const void *)diff_forward_kernel<kPackedNormals>
+           : source == kPackedQuads ? (const void *)diff_forward_kernel<kPackedQuads>
+                                    : (const void *)diff_forward_kernel<kLinear>;
+}
+
+template <bool WARP_TABLE>
+const void *backward_kernel(int source) {
+    return source == kPackedNormals ? (const void *)diff_backward_kernel<kPackedNormals, WARP_TABLE>
+           : source == kPackedQuads ? (const void *)diff_backward_kernel<kPackedQuads, WARP_TABLE>
+                                    : (const void *)diff_backward_kernel<kLinear, WARP_TABLE>;
+}
+
 }  // namespace
 }  // namespace pvr
 
 using pvr::fail;
 
-extern "C" int pvr_diff_forward(const pvr_diff_scene *s, float *d_image, int *d_steps, void *stream) {
+extern "C" int pvr_diff_workspace(const pvr_diff_scene *s, long long *bytes, long long *bytes_volume_gradient) {
+    if (!bytes || !bytes_volume_gradient) return fail(PVR_ERR_VALUE, "bytes is NULL");
+    *bytes = *bytes_volume_gradient = 0;
+    if (int rc = pvr::check_scene(s)) return rc;
+    *bytes = pvr::packed_bytes(s, s->normals != nullptr);
+    *bytes_volume_gradient = *bytes > 0 ? *bytes + pvr::packed_bytes(s, false) : 0;
+    return PVR_OK;
+}
+
+extern "C" int pvr_diff_forward_ws(const pvr_diff_scene *s, float *d_image, int *d_steps, void *workspace,
+                                   long long workspace_bytes, void *stream) {
     if (int rc = pvr::check_scene(s)) return rc;
     if (!d_image || !d_steps) return fail(PVR_ERR_VALUE, "image / steps buffer is NULL");
+    if (int rc = pvr::check_workspace(workspace, workspace_bytes)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    const long long frame = (long long)s->width * s->height;
+    pvr::Packed packed;
+    for (int v0 = 0; v0 < s->n_views; v0 += pvr::kDiffMaxViews) {
+        const int nv = std::min(pvr::kDiffMaxViews, s->n_views - v0);
+        pvr::DiffParams p;
+        if (int rc = pvr::build_params(s, v0, nv, p)) return rc;
+        if (v0 == 0) PVR_CUDA(pvr::pack_scene(s, false, workspace, workspace_bytes, st, packed));
+        p.texels = packed.texels;
+        p.image = reinterpret_cast<float4 *>(d_image) + v0 * frame;
+        p.steps = d_steps + v0 * frame;
+        const int blocks = p.tiles_x * p.tiles_y * nv;
+        void *args[] = {&p};
+        PVR_CUDA(cudaLaunchKernel(pvr::forward_kernel(packed.source), dim3(blocks), dim3(pvr::kDiffThreads), args,
+                                  (size_t)(s->lut_size + 2) * sizeof(float4), st));
+    }
+    return PVR_OK;
+}
+
+extern "C" int pvr_diff_forward(const pvr_diff_scene *s, float *d_image, int *d_steps, void *stream) {
+    return pvr_diff_forward_ws(s, d_image, d_steps, nullptr, 0, stream);
+}
+
+extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_image, const int *d_steps,
+                                    const float *d_grad_image, float *d_grad_lut, float *d_grad_volume,
+                                    void *workspace, long long workspace_bytes, void *stream) {
+    if (int rc = pvr::check_scene(s)) return rc;
+    if (!d_image || !d_steps || !d_grad_image) return fail(PVR_ERR_VALUE, "image / steps / gradient buffer is NULL");
+    if (int rc = pvr::check_workspace(workspace, workspace_bytes)) return rc;
+    if (!d_grad_lut && !d_grad_volume) return PVR_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    int device = 0, sms = 0;
+    PVR_CUDA(cudaGetDevice(&device));
+    PVR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const bool warp_table = s->lut_size <= pvr::kWarpTableLut;
+    const size_t rows = (size_t)s->lut_size + 2;
+    const size_t smem = rows * sizeof(float4) * (d_grad_lut ? (warp_table ? 1 + pvr::kDiffThreads / 32 : 2) : 1);
+    int per_sm = 0;
+    pvr::Packed packed;
+    const void *kernel = nullptr;
     const long long frame = (long long)s->width * s->height;
     for (int v0 = 0; v0 < s->n_views; v0 += pvr::kDiffMaxViews) {
         const int nv = std::min(pvr::kDiffMaxViews, s->n_views - v0);
         pvr::DiffParams p;
         if (int rc = pvr::build_params(s, v0, nv, p)) return rc;
-        p.image = reinterpret_cast<float4 *>(d_image) + v0 * frame;
-        p.steps = d_steps + v0 * frame;
-        const int blocks = p.tiles_x * p.tiles_y * nv;
+        if (v0 == 0) {
+            PVR_CUDA(pvr::pack_scene(s, d_grad_volume != nullptr, workspace, workspace_bytes, st, packed));
+            kernel = warp_table ? pvr::backward_kernel<true>(packed.source) : pvr::backward_kernel<false>(packed.source);
+            // more than 48 KB of dynamic shared memory (set on the current device)
+            if (smem > 48 * 1024)
+                PVR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PVR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, pvr::kDiffThreads, smem));
+            per_sm = std::max(1, per_sm);
+        }
+        p.texels = packed.texels;
+        p.image = const_cast<float4 *>(reinterpret_cast<const float4 *>(d_image)) + v0 * frame;
+        p.steps = const_cast<int *>(d_steps) + v0 * frame;
+        p.gimage = reinterpret_cast<const float4 *>(d_grad_image) + v0 * frame;
+        p.glut = reinterpret_cast<float4 *>(d_grad_lut);
+        p.gvol = d_grad_volume;
+        p.gquads = packed.gquads;
+        const int tiles = p.tiles_x * p.tiles_y * nv;
+        const int blocks = std::min(tiles, sms * per_sm);
         void *args[] = {&p};
-        PVR_CUDA(cudaLaunchKernel((const void *)pvr::diff_forward_kernel, dim3(blocks), dim3(pvr::kDiffThreads),
-                                  args, 0, st));
+        PVR_CUDA(cudaLaunchKernel(kernel, dim3(blocks), dim3(pvr::kDiffThreads), args, smem, st));
+    }
+    if (packed.gquads) {
+        const int voxels = s->d * s->h * s->w;
+        pvr::unpack_grad_kernel<<<(voxels + 255) / 256, 256, 0, st>>>(packed.gquads, s->w, s->h, s->d, d_grad_volume);
+        PVR_CUDA(cudaGetLastError());
     }
     return PVR_OK;
 }
@@ -471,38 +746,5 @@ extern "C" int pvr_diff_forward(const pvr_diff_scene *s, float *d_image, int *d_
 extern "C" int pvr_diff_backward(const pvr_diff_scene *s, const float *d_image, const int *d_steps,
                                  const float *d_grad_image, float *d_grad_lut, float *d_grad_volume,
                                  void *stream) {
-    if (int rc = pvr::check_scene(s)) return rc;
-    if (!d_image || !d_steps || !d_grad_image) return fail(PVR_ERR_VALUE, "image / steps / gradient buffer is NULL");
-    if (!d_grad_lut && !d_grad_volume) return PVR_OK;
-    cudaStream_t st = (cudaStream_t)stream;
-    int device = 0, sms = 0;
-    PVR_CUDA(cudaGetDevice(&device));
-    PVR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const size_t smem = (size_t)pvr::kSeg * 3 * pvr::kDiffThreads * sizeof(float) +
-                        (d_grad_lut ? (size_t)s->lut_size * 4 * sizeof(float) : 0);
-    // more than 48 KB of dynamic shared memory (set on the current device)
-    PVR_CUDA(cudaFuncSetAttribute((const void *)pvr::diff_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(pvr::kSeg * 3 * pvr::kDiffThreads * sizeof(float) +
-                                        pvr::kDiffMaxLut * 4 * sizeof(float))));
-    int per_sm = 0;
-    PVR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pvr::diff_backward_kernel, pvr::kDiffThreads,
-                                                           smem));
-    per_sm = std::max(1, per_sm);
-    const long long frame = (long long)s->width * s->height;
-    for (int v0 = 0; v0 < s->n_views; v0 += pvr::kDiffMaxViews) {
-        const int nv = std::min(pvr::kDiffMaxViews, s->n_views - v0);
-        pvr::DiffParams p;
-        if (int rc = pvr::build_params(s, v0, nv, p)) return rc;
-        p.image = const_cast<float4 *>(reinterpret_cast<const float4 *>(d_image)) + v0 * frame;
-        p.steps = const_cast<int *>(d_steps) + v0 * frame;
-        p.gimage = reinterpret_cast<const float4 *>(d_grad_image) + v0 * frame;
-        p.glut = reinterpret_cast<float4 *>(d_grad_lut);
-        p.gvol = d_grad_volume;
-        const int tiles = p.tiles_x * p.tiles_y * nv;
-        const int blocks = std::min(tiles, sms * per_sm);
-        void *args[] = {&p};
-        PVR_CUDA(cudaLaunchKernel((const void *)pvr::diff_backward_kernel, dim3(blocks), dim3(pvr::kDiffThreads),
-                                  args, smem, st));
-    }
-    return PVR_OK;
+    return pvr_diff_backward_ws(s, d_image, d_steps, d_grad_image, d_grad_lut, d_grad_volume, nullptr, 0, stream);
 }

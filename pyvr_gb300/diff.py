@@ -3,10 +3,9 @@ RGBA transfer-function LUT and the voxel values, from a hand-written CUDA
 backward (``pvr_diff_backward``) behind ``torch.autograd.Function``.
 
 The forward is the renderer's march (pyvr/shaders/volume.frag.glsl:70-122)
-over an FP32 volume in its (D, H, W) layout, for several views of one scene
-at once; its float image is the renderer's float image bit for bit.  The
-backward marches each ray a second time in reverse and rebuilds the
-transmittance from the final alpha (T_i = T_{i+1} / (1 - alpha_i)), so no
+over an FP32 volume, for several views of one scene at once; its float image
+is the renderer's float image bit for bit.  The backward marches each ray a
+second time and takes what lies behind a sample from the image, so no
 per-sample state is stored: only the loop length of each pixel.  Normals (a
 given normal volume, or none) are constants of the scene.
 
@@ -94,6 +93,20 @@ def _check_inputs(volume, lut, normals):
         raise ValueError("volume, lut and normals must be on one device")
 
 
+def _workspace(nbytes: int, device):
+    """Scratch tensor in which a call packs the scene's texels, or None where
+    that does not pay (0 bytes) or the memory is not there (the call then
+    reads the scene's own arrays)."""
+    import torch
+    if nbytes == 0:
+        return None, None, 0
+    try:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None, None, 0
+    return ws, ws.data_ptr(), nbytes
+
+
 def _march_function():
     import torch
 
@@ -109,8 +122,13 @@ def _march_function():
             steps = torch.empty((v, h, w), dtype=torch.int32, device=volume.device)
             c = scene.c_scene(volume, lut, normals)
             stream = torch.cuda.current_stream(volume.device).cuda_stream
-            check(_lib().pvr_diff_forward(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), stream))
+            n, n_vol = ctypes.c_longlong(0), ctypes.c_longlong(0)
+            check(_lib().pvr_diff_workspace(ctypes.byref(c), ctypes.byref(n), ctypes.byref(n_vol)))
+            ws = _workspace(n.value, volume.device)
+            check(_lib().pvr_diff_forward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), ws[1], ws[2],
+                                             stream))
             ctx.scene = scene
+            ctx.workspace_bytes = (n.value, n_vol.value)
             ctx.save_for_backward(volume, lut, normals, image, steps)
             ctx.mark_non_differentiable(steps)
             return image, steps
@@ -125,9 +143,11 @@ def _march_function():
                 gimage = gimage.contiguous()
                 c = ctx.scene.c_scene(volume, lut, normals)
                 stream = torch.cuda.current_stream(volume.device).cuda_stream
-                check(_lib().pvr_diff_backward(ctypes.byref(c), image.data_ptr(), steps.data_ptr(),
-                                               gimage.data_ptr(), glut.data_ptr() if glut is not None else None,
-                                               gvol.data_ptr() if gvol is not None else None, stream))
+                ws = _workspace(ctx.workspace_bytes[1 if need_vol else 0], volume.device)
+                check(_lib().pvr_diff_backward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(),
+                                                  gimage.data_ptr(), glut.data_ptr() if glut is not None else None,
+                                                  gvol.data_ptr() if gvol is not None else None, ws[1], ws[2],
+                                                  stream))
             return gvol, glut, None, None
 
     return _March

@@ -171,3 +171,53 @@ def test_adam_recovers_transfer_function():
             lut.clamp_(0.0, 1.0)
         losses.append(loss.item())
     assert losses[-1] < 0.3 * losses[0], losses
+
+
+@pytest.mark.parametrize("dims,lut_size,normals,opaque", [
+    ((6, 11, 9), 1, True, False), ((6, 11, 9), 2, False, False), ((2, 17, 3), 512, True, True),
+    ((1, 5, 8), 513, False, False), ((13, 2, 1), 2048, False, True), ((33, 16, 31), 777, True, False)])
+def test_packed_texels_and_tables_at_their_edges(dims, lut_size, normals, opaque):
+    # odd and thin volumes, tables of one entry, on both sides of the per-warp
+    # gradient table's limit and of the largest size; opaque: some entries have
+    # alpha exactly 1 after the opacity correction
+    rng = np.random.default_rng(11)
+    data = rng.random(dims, dtype=np.float32) * 1.2 - 0.1  # below and above the table too
+    nrm = rng.normal(size=dims + (3,)).astype(np.float32) if normals else None
+    lut = np.concatenate([rng.random((lut_size, 3)), rng.uniform(0.0, 0.2, (lut_size, 1))], 1).astype(np.float32)
+    if opaque:
+        lut[lut_size // 2:, 3] = 200.0
+    w, h = 37, 29
+    cams = [Camera.from_spherical(np.zeros(3, np.float32), a, 0.4, 0.0, 3.0) for a in (0.3, 2.1)]
+    light, cfg = Light.directional([1, -1, 0], 0.2, 0.8), RenderConfig.fast()
+    scene = DiffScene(cams, light, cfg, w, h)
+    vol = Volume(data=data, normals=nrm, min_bounds=np.full(3, -1.0, np.float32),
+                 max_bounds=np.full(3, 1.0, np.float32))
+    frames = [W.frame_inputs(vol, c, light, cfg, lut, w, h) for c in cams]
+    target = torch.tensor(rng.random((2, h, w, 4), dtype=np.float32))
+    gv, gl = _dev(data, True), _dev(lut, True)
+    img = render_views(gv, gl, scene, _dev(nrm) if normals else None)
+    for k, s in enumerate(frames):
+        assert np.array_equal(img[k].detach().cpu().numpy().view(np.uint32), oracle.render(s)[1].view(np.uint32)), k
+    ((img - target.cuda()) ** 2).mean().backward()
+    tv, tl = torch.tensor(data, requires_grad=True), torch.tensor(lut, requires_grad=True)
+    ref, _ = march_torch.render_views(tv, tl, frames, torch.tensor(nrm) if normals else None, torch.float32)
+    ((ref - target) ** 2).mean().backward()
+    # the tolerances of test_backward_matches_torch_autograd
+    for name, gk, gt in (("lut", gl.grad, tl.grad), ("volume", gv.grad, tv.grad)):
+        gk, gt = gk.cpu().numpy(), gt.numpy()
+        assert np.linalg.norm(gk - gt) <= 2e-3 * np.linalg.norm(gt), name
+        assert np.abs(gk - gt).max() <= 1e-2 * np.abs(gt).max(), name
+
+
+def test_scenes_without_packing_render_the_same():
+    # a large volume for few pixels is read from its own arrays
+    c = _case(n=48, res=8, views=1)
+    vol, lut, nrm = _dev(c["data"], True), _dev(c["lut0"], True), _dev(c["nrm"])
+    img = render_views(vol, lut, c["scene"], nrm)
+    assert np.array_equal(img[0].detach().cpu().numpy().view(np.uint32), oracle.render(c["frames"][0])[1].view(np.uint32))
+    img.square().mean().backward()
+    tv, tl = torch.tensor(c["data"], requires_grad=True), torch.tensor(c["lut0"], requires_grad=True)
+    ref, _ = march_torch.render_views(tv, tl, c["frames"], torch.tensor(c["nrm"]), torch.float32)
+    ref.square().mean().backward()
+    for gk, gt in ((lut.grad, tl.grad), (vol.grad, tv.grad)):
+        assert (gk.cpu() - gt).norm() <= 2e-3 * gt.norm()
