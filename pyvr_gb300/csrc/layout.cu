@@ -15,11 +15,11 @@
 // records, and the 8 texels of a sample sit at fixed offsets from one
 // record address.  Bricks are stored in Morton order of their brick
 // coordinates (a warp's rays walk neighbouring bricks, which then sit in
-// neighbouring memory), located through a brick table.  A per-brick
+// neighbouring memory), located through the brick array.  A per-brick
 // min/max of the stored values lets the march skip bricks that the current
 // LUT makes exactly transparent.
 #include <algorithm>
-#include <vector>
+#include <cstring>
 
 #include "normals.cuh"
 #include "pvr_device.cuh"
@@ -39,26 +39,6 @@ template <> __device__ __forceinline__ float raw_value<__half>(const __half *p, 
 }
 
 
-// The normal of array element (a, b, c), its neighbours read from global
-// memory.
-template <typename T>
-__device__ float3 normal_global(const T *v, const int dims[3], int a, int b, int c) {
-    const int idx[3] = {a, b, c};
-    const long long stride[3] = {(long long)dims[1] * dims[2], dims[2], 1};
-    const long long base = a * stride[0] + b * stride[1] + c;
-    float g[3];
-    const float v0 = raw_value<T>(v, base);
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        const int i = idx[ax], n = dims[ax];
-        const long long s = stride[ax];
-        const float vm = i > 0 ? raw_value<T>(v, base - s) : 0.0f;
-        const float vp = i < n - 1 ? raw_value<T>(v, base + s) : 0.0f;
-        g[ax] = GradientArith<T>::axis(vm, v0, vp, i, n);
-    }
-    return GradientArith<T>::finish(g[0], g[1], g[2]);
-}
-
 template <typename Rec> __device__ __forceinline__ Rec make_record(float v, float3 n);
 template <> __device__ __forceinline__ float4 make_record<float4>(float v, float3 n) {
     return make_float4(v, n.x, n.y, n.z);
@@ -70,108 +50,380 @@ template <> __device__ __forceinline__ uint2 make_record<uint2>(float v, float3 
     return make_uint2(h0 | (h1 << 16), h2 | (h3 << 16));
 }
 
+// One record's slot: the rank of the brick's Morton code (x, y, z interleaved,
+// x first) among the codes of the brick grid.  Walking down the octree, the
+// codes before this one at a level are those of the children in front of the
+// brick's own child, each a box whose part inside the grid is a product of
+// three extents.  (Sorting the codes on the host took 1 ms for 33^3 bricks
+// and delayed the upload; this is one thread per brick.)
+__device__ __forceinline__ long long inside(int o, int h, int n) { return min(max(n - o, 0), h); }
+
+__global__ void brick_slots_kernel(BrickGeometry g, uint4 *__restrict__ bricks) {
+    const int brick = blockIdx.x * blockDim.x + threadIdx.x;
+    if (brick >= g.nbricks) return;
+    const int b[3] = {brick / (g.nb[2] * g.nb[1]), (brick / g.nb[2]) % g.nb[1], brick % g.nb[2]};
+    int o[3] = {0, 0, 0};
+    long long before = 0;
+    const int top = 31 - __clz(max(max(g.nb[0], g.nb[1]), g.nb[2]));
+    for (int level = top; level >= 0; --level) {
+        const int h = 1 << level;
+        long long lo[3], own[3], all[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = inside(o[a], h, g.nb[a]);
+            const long long hi = inside(o[a] + h, h, g.nb[a]);
+            const bool up = (b[a] >> level) & 1;
+            own[a] = up ? hi : lo[a];
+            all[a] = lo[a] + hi;
+            lo[a] = up ? lo[a] : 0;  // the half in front of the own one
+            if (up) o[a] += h;
+        }
+        before += lo[0] * all[1] * all[2] + own[0] * (lo[1] * all[2] + own[1] * lo[2]);
+    }
+    bricks[brick].x = (uint32_t)before;
+}
+
+// Records of one storage type, built in groups of kStep along x: float one by
+// one; uint8 and float16, whose values are halves exactly, in pairs of halves.
+template <typename T> struct Lanes;
+
+template <> struct Lanes<float> {
+    static constexpr int kStep = 1;
+    using Word = float;
+    static __device__ __forceinline__ float load(const float *p) { return __ldg(p); }
+    static __device__ __forceinline__ Word word(float cur, float) { return cur; }
+    // the word of two texels taken from the low lanes of two words
+    static __device__ __forceinline__ Word join(Word a, Word) { return a; }
+    static __device__ __forceinline__ Word diff(Word p, Word m) { return __fsub_rn(p, m); }
+    static __device__ __forceinline__ Word scaled(Word d, Word s) { return __fmul_rn(d, s); }
+    static __device__ __forceinline__ Word scales(float a, float) { return a; }
+    static __device__ __forceinline__ void range(Word w, bool, Word &lo, Word &hi) {
+        lo = fminf(lo, w);
+        hi = (w != w || hi != hi) ? w + hi : fmaxf(hi, w);  // NaN sticks
+    }
+    static __device__ __forceinline__ Word lo_start() { return __int_as_float(0x7f800000); }
+    static __device__ __forceinline__ Word hi_start() { return -__int_as_float(0x7f800000); }
+    static __device__ __forceinline__ float lo_float(Word w) { return w; }
+    static __device__ __forceinline__ float hi_float(Word w) { return w; }
+    static __device__ __forceinline__ void records(Word v, Word g0, Word g1, Word g2, bool normals, float4 *out,
+                                                   int, bool) {
+        const float3 n = normals ? GradientArith<float>::finish(g0, g1, g2) : make_float3(0.0f, 0.0f, 0.0f);
+        *out = make_float4(v, n.x, n.y, n.z);
+    }
+};
+
+__device__ __forceinline__ __half2 halves(uint32_t u) {
+    __half2 h;
+    memcpy(&h, &u, sizeof(h));
+    return h;
+}
+
+struct HalfLanes {
+    static constexpr int kStep = 2;
+    using Word = uint32_t;
+    static __device__ __forceinline__ Word join(Word a, Word b) { return __byte_perm(a, b, 0x5410); }
+    static __device__ __forceinline__ Word diff(Word p, Word m) { return half_bits(__hsub2(halves(p), halves(m))); }
+    static __device__ __forceinline__ Word scaled(Word d, Word s) { return half_bits(__hmul2(halves(d), halves(s))); }
+    static __device__ __forceinline__ Word scales(float a, float b) { return half_bits(__floats2half2_rn(a, b)); }
+    static __device__ __forceinline__ void range(Word w, bool both, Word &lo, Word &hi) {
+        const __half2 v = halves(both ? w : __byte_perm(w, w, 0x1010));
+        lo = half_bits(__hmin2(halves(lo), v));
+        hi = half_bits(__hmax2_nan(halves(hi), v));  // NaN sticks
+    }
+    static __device__ __forceinline__ Word lo_start() { return 0x7c007c00u; }
+    static __device__ __forceinline__ Word hi_start() { return 0xfc00fc00u; }
+    static __device__ __forceinline__ float lo_float(Word w) {
+        const float2 f = __half22float2(halves(w));
+        return fminf(f.x, f.y);
+    }
+    static __device__ __forceinline__ float hi_float(Word w) {
+        const float2 f = __half22float2(halves(w));
+        return (f.x != f.x || f.y != f.y) ? f.x + f.y : fmaxf(f.x, f.y);
+    }
+    // two half records `stride` apart: component words {n(x), n(x + 1)}
+    static __device__ __forceinline__ void store(Word v, Word n0, Word n1, Word n2, uint2 *out, int stride, bool both) {
+        out[0] = make_uint2(__byte_perm(v, n0, 0x5410), __byte_perm(n1, n2, 0x5410));
+        if (both) out[stride] = make_uint2(__byte_perm(v, n0, 0x7632), __byte_perm(n1, n2, 0x7632));
+    }
+};
+
+template <> struct Lanes<__half> : HalfLanes {
+    static __device__ __forceinline__ uint32_t load(const __half *p) {
+        return __ldg(reinterpret_cast<const unsigned short *>(p));
+    }
+    static __device__ __forceinline__ Word word(uint32_t cur, uint32_t next) { return cur | (next << 16); }
+    static __device__ __forceinline__ void normals(Word g0, Word g1, Word g2, Word n[3]) {
+        const __half2 g[3] = {halves(g0), halves(g1), halves(g2)};
+        __half2 h[3];
+        if (f16_halves(g[0], g[1], g[2], h)) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) n[a] = half_bits(h[a]);
+        } else {  // a flat place (0 / 0 = NaN, g / 0 = inf, as numpy has it), or infinities
+            const float2 ss = f16_square_sum(g[0], g[1], g[2]);
+            const float2 len = __half22float2(__floats2half2_rn(__fsqrt_rn(ss.x), __fsqrt_rn(ss.y)));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float2 f = __half22float2(g[a]);
+                n[a] = half_bits(__floats2half2_rn(__fdiv_rn(f.x, len.x), __fdiv_rn(f.y, len.y)));
+            }
+        }
+    }
+    static __device__ __forceinline__ void records(Word v, Word g0, Word g1, Word g2, bool with, uint2 *out, int stride,
+                                                   bool both) {
+        Word n[3] = {0u, 0u, 0u};
+        if (with) normals(g0, g1, g2, n);
+        store(v, n[0], n[1], n[2], out, stride, both);
+    }
+    static __device__ __forceinline__ void records(Word v, Word g0, Word g1, Word g2, bool with, float4 *out,
+                                                   int stride, bool both) {
+        Word n[3] = {0u, 0u, 0u};
+        if (with) normals(g0, g1, g2, n);
+        const float2 f = __half22float2(halves(v)), a = __half22float2(halves(n[0])), b = __half22float2(halves(n[1])),
+                     c = __half22float2(halves(n[2]));
+        out[0] = make_float4(f.x, a.x, b.x, c.x);
+        if (both) out[stride] = make_float4(f.y, a.y, b.y, c.y);
+    }
+};
+
+template <> struct Lanes<uint8_t> : HalfLanes {
+    static __device__ __forceinline__ uint32_t load(const uint8_t *p) { return __ldg(p); }
+    // 1024 + u is the half with u in its low mantissa bits
+    static __device__ __forceinline__ Word word(uint32_t cur, uint32_t next) {
+        return half_bits(__hsub2(halves(cur | (next << 16) | 0x64006400u), halves(0x64006400u)));
+    }
+    static __device__ __forceinline__ void records(Word v, Word g0, Word g1, Word g2, bool with, uint2 *out, int stride,
+                                                   bool both) {
+        Word n[3] = {0u, 0u, 0u};
+        if (with) {
+            const float2 a = __half22float2(halves(g0)), b = __half22float2(halves(g1)), c = __half22float2(halves(g2));
+            __half2 h[3];
+            if (!u8_halves(a, b, c, h)) {
+                const float3 p = GradientArith<uint8_t>::finish(a.x, b.x, c.x);
+                const float3 q = GradientArith<uint8_t>::finish(a.y, b.y, c.y);
+                h[0] = __floats2half2_rn(p.x, q.x);
+                h[1] = __floats2half2_rn(p.y, q.y);
+                h[2] = __floats2half2_rn(p.z, q.z);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) n[k] = half_bits(h[k]);
+        }
+        store(v, n[0], n[1], n[2], out, stride, both);
+    }
+    static __device__ __forceinline__ void records(Word v, Word g0, Word g1, Word g2, bool with, float4 *out,
+                                                   int stride, bool both) {
+        const float2 f = __half22float2(halves(v)), a = __half22float2(halves(g0)), b = __half22float2(halves(g1)),
+                     c = __half22float2(halves(g2));
+        const float3 zero = make_float3(0.0f, 0.0f, 0.0f);
+        const float3 p = with ? GradientArith<uint8_t>::finish(a.x, b.x, c.x) : zero;
+        out[0] = make_float4(f.x, p.x, p.y, p.z);
+        if (!both) return;
+        const float3 q = with ? GradientArith<uint8_t>::finish(a.y, b.y, c.y) : zero;
+        out[stride] = make_float4(f.y, q.x, q.y, q.z);
+    }
+};
+
+template <int LOG2B> struct BrickShape {
+    static constexpr int B = 1 << LOG2B, A = B + 1, Q = A * A, S = B + 3, P = S * S;
+    // one thread per (y, z) of a slice of records; 16^3 bricks: 289 of 320
+    static constexpr int kThreads = LOG2B == 4 ? 320 : LOG2B == 3 ? 128 : 64;
+};
+
+// Writes a brick's {min, max} from the threads' own (a NaN maximum marks the
+// brick as never skippable).  All threads of the block call it.
+template <int THREADS>
+__device__ __forceinline__ void write_range(float lo, float hi, uint4 *brick) {
+    __shared__ float s_lo[THREADS / 32], s_hi[THREADS / 32];
+    __shared__ int s_nan[THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool nan = __any_sync(0xffffffffu, hi != hi);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+        s_lo[warp] = lo;
+        s_hi[warp] = hi;
+        s_nan[warp] = nan;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bool any_nan = false;
+        for (int w = 0; w < THREADS / 32; ++w) {
+            lo = fminf(lo, s_lo[w]);
+            hi = fmaxf(hi, s_hi[w]);
+            any_nan |= s_nan[w] != 0;
+        }
+        brick->y = any_nan ? 0x7fc00000u : __float_as_uint(lo);
+        brick->z = any_nan ? 0u : __float_as_uint(hi);
+        brick->w = 0u;
+    }
+}
+
+// The layout of volumes without normals, and of cubic volumes (array axes =
+// world axes) with device normals (numpy.gradient semantics).  One block per
+// brick, bricks [brick0, brick0 + gridDim.x) in x-major order.
+//
+// What bounds it: the instructions per record (the earlier kernel issued on
+// 90 % of cycles at 353 of them; DRAM 11 %).  So a thread owns one (y, z)
+// of the brick and walks x: all its indices are set up once, the texels of a
+// slice and of the next one are fixed offsets apart, and the x neighbour of
+// one step is the one of the step after next.  uint8 and float16 texels are
+// staged as pairs of halves {x, x + 1}, so that one packed instruction does
+// two records.  NORMALS: compute them (else zero).  Records of a slice are
+// stored contiguously by neighbouring threads.  Voxel (x, y, z) along world
+// axes lives at z + D*(y + H*x) of the (D,H,W) C-order buffer (the GL texture
+// of size (D,H,W) read through the z/y/x swizzle, volume.frag.glsl:90).
+// Measured: 512^3 in 33^3 bricks of 17^3 half records, float16 1720 -> 557 us,
+// uint8 1722 -> 457 us; 256^3 in bricks of 9^3 float records, uint8 338 -> 152 us,
+// float32 249 -> 121 us.  16^3 bricks: 4 blocks per SM (48 registers); at 3 (64
+// registers, float16 796 us) and 5 (32, spills, 744 us) it is slower.
+template <typename T, int LOG2B, typename Rec, bool NORMALS>
+__global__ void __launch_bounds__(BrickShape<LOG2B>::kThreads, LOG2B == 4 ? 4 : 1)
+build_walk_kernel(BrickGeometry g, const T *__restrict__ vol, int brick0, Rec *__restrict__ records,
+                  uint4 *__restrict__ bricks) {
+    using Sh = BrickShape<LOG2B>;
+    using L = Lanes<T>;
+    using Word = typename L::Word;
+    constexpr int B = Sh::B, A = Sh::A, Q = Sh::Q, S = Sh::S, P = Sh::P;
+    __shared__ Word sw[S * P];
+    const int brick = brick0 + blockIdx.x;
+    const int bz = brick % g.nb[2], by = (brick / g.nb[2]) % g.nb[1], bx = brick / (g.nb[2] * g.nb[1]);
+    // staged texels: b*B - 2 + r on each axis, r in [0, S), clamped to the
+    // volume; word (rx, ry, rz) holds texel rx and, in pairs, texel rx + 1
+    const int ox = bx * B - 2, oy = by * B - 2, oz = bz * B - 2;
+    const uint32_t slice = (uint32_t)g.ext[1] * (uint32_t)g.ext[2];
+    for (int q = threadIdx.x; q < P; q += Sh::kThreads) {
+        const int y = min(max(oy + q / S, 0), g.ext[1] - 1), z = min(max(oz + q % S, 0), g.ext[2] - 1);
+        const T *src = vol + ((uint32_t)y * (uint32_t)g.ext[2] + (uint32_t)z);
+        auto at = [&](int r) { return L::load(src + (uint32_t)min(max(ox + r, 0), g.ext[0] - 1) * (size_t)slice); };
+        auto cur = at(0);
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+            const auto next = r + 1 < S && L::kStep == 2 ? at(r + 1) : cur;
+            sw[r * P + q] = L::word(cur, next);
+            cur = L::kStep == 2 ? next : (r + 1 < S ? at(r + 1) : cur);
+        }
+    }
+    __syncthreads();
+    Word lo = L::lo_start(), hi = L::hi_start();
+    const uint32_t slot = bricks[brick].x;
+    Rec *out = records + (size_t)slot * brick_records(LOG2B) + threadIdx.x;
+    if (threadIdx.x < Q) {
+        const int ly = threadIdx.x / A, lz = threadIdx.x % A;
+        // local indices of the volume's first and last texel: record l holds
+        // texel clamp(b*B - 1 + l)
+        const int fx = bx == 0 ? 1 : -9, fy = by == 0 ? 1 : -9, fz = bz == 0 ? 1 : -9;
+        const int ex = g.ext[0] - bx * B, ey = g.ext[1] - by * B, ez = g.ext[2] - bz * B;
+        if (fx < 0 && fy < 0 && fz < 0 && ex > B && ey > B && ez > B) {
+            // every record and every neighbour lies inside the volume
+            const Word *c = sw + (S + ly + 1) * S + lz + 1;
+            Word xm = c[-P];
+            const Word half = L::scales(0.5f, 0.5f);
+#pragma unroll
+            for (int l = 0; l < A; l += L::kStep, c += L::kStep * P, out += L::kStep * Q) {
+                const Word v = c[0], xp = c[P];
+                const bool both = l + 1 < A;
+                L::range(v, both, lo, hi);
+                Word g0 = 0, g1 = 0, g2 = 0;
+                if (NORMALS) {
+                    g0 = L::scaled(L::diff(xp, xm), half);
+                    g1 = L::scaled(L::diff(c[S], c[-S]), half);
+                    g2 = L::scaled(L::diff(c[1], c[-1]), half);
+                    xm = L::kStep == 2 ? xp : v;
+                }
+                L::records(v, g0, g1, g2, NORMALS, out, Q, both);
+            }
+        } else {
+            // a brick at the volume's faces: clamped texels, and one-sided
+            // differences on them
+            auto clampl = [](int l, int f, int e) { return min(max(l, f), e); };
+            const int y = clampl(ly, fy, ey), z = clampl(lz, fz, ez);
+            const int ym = y == fy ? y : y - 1, yp = y == ey ? y : y + 1;
+            const int zm = z == fz ? z : z - 1, zp = z == ez ? z : z + 1;
+            const float hy = ym == y || yp == y ? 1.0f : 0.5f, hz = zm == z || zp == z ? 1.0f : 0.5f;
+            const Word sy = L::scales(hy, hy), sz = L::scales(hz, hz);
+            auto at = [&](int xa, int xb, int yy, int zz) {
+                const int o = (yy + 1) * S + zz + 1;
+                return L::join(sw[(xa + 1) * P + o], sw[(xb + 1) * P + o]);
+            };
+            for (int l = 0; l < A; l += L::kStep, out += L::kStep * Q) {
+                const bool both = l + 1 < A;
+                const int xa = clampl(l, fx, ex), xb = clampl(min(l + 1, A - 1), fx, ex);
+                const Word v = at(xa, xb, y, z);
+                L::range(v, true, lo, hi);
+                Word g0 = 0, g1 = 0, g2 = 0;
+                if (NORMALS) {
+                    const bool fa = xa == fx || xa == ex, fb = xb == fx || xb == ex;
+                    g0 = L::scaled(L::diff(at(xa == ex ? xa : xa + 1, xb == ex ? xb : xb + 1, y, z),
+                                           at(xa == fx ? xa : xa - 1, xb == fx ? xb : xb - 1, y, z)),
+                                   L::scales(fa ? 1.0f : 0.5f, fb ? 1.0f : 0.5f));
+                    g1 = L::scaled(L::diff(at(xa, xb, yp, z), at(xa, xb, ym, z)), sy);
+                    g2 = L::scaled(L::diff(at(xa, xb, y, zp), at(xa, xb, y, zm)), sz);
+                }
+                L::records(v, g0, g1, g2, NORMALS, out, Q, both);
+            }
+        }
+    }
+    write_range<Sh::kThreads>(L::lo_float(lo), L::hi_float(hi), bricks + brick);
+}
+
 constexpr int kLayoutThreads = 256;
 
-// One block per brick (grid-stride over bricks; launched with one block per
-// brick).  The block first stages
-// the brick's texels plus a two-texel margin ((B+3)^3, clamped to the
-// volume) in shared memory, then writes the brick's (B+1)^3 records: the
-// stored value and the normal (given: read from `nrm`; computed on the
-// device: numpy.gradient from the staged neighbours when the volume is
-// cubic -- array axes are then the world axes -- else from global memory),
-// and finally the brick's {slot, min, max} from a block reduction over the
-// records' values (a NaN marks the brick as never skippable).  Voxel
-// (x, y, z) along world axes lives at z + D*(y + H*x) of the (D,H,W) C-order
-// buffer (the GL texture of size (D,H,W) read through the z/y/x swizzle,
-// volume.frag.glsl:90); the normal texture is indexed the same way
-// (manager.py:123-125).  Rec: float4 records, or uint2 half records (only
-// for storage types whose values are halves exactly).
+// n / d for n < 2^31 by one multiplication (Granlund & Montgomery 1994).
+struct FastDiv {
+    uint32_t d, m, s;
+    explicit FastDiv(uint32_t div) : d(div), s(0) {
+        while ((1ull << s) < d) ++s;
+        m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+    }
+    __device__ __forceinline__ uint32_t quot(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
+};
+
+// The layout of the other volumes: given normals (read from `nrm`, indexed
+// like the voxels: manager.py:123-125), and device normals of non-cubic
+// volumes, whose array axes are not the world axes (the neighbours come from
+// global memory).  One block per brick; a thread per record.
 template <typename T, int LOG2B, typename Rec>
 __global__ void __launch_bounds__(kLayoutThreads)
-build_bricks_kernel(BrickGeometry g, const T *__restrict__ vol, int D, int H, int W,
-                    const float *__restrict__ nrm, int normals_mode, const uint32_t *__restrict__ table,
-                    Rec *__restrict__ records, uint4 *__restrict__ bricks) {
-    constexpr int B = 1 << LOG2B, A = B + 1, R = A * A * A, S = B + 3, S3 = S * S * S;
-    constexpr int WARPS = kLayoutThreads / 32;
-    __shared__ float sv[S3];
-    __shared__ float s_lo[WARPS], s_hi[WARPS];
-    __shared__ int s_nan[WARPS];
-    const int dims[3] = {D, H, W};
-    const bool cubic = D == H && H == W;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int brick = blockIdx.x; brick < g.nbricks; brick += gridDim.x) {
-        const int bz = brick % g.nb[2];
-        const int by = (brick / g.nb[2]) % g.nb[1];
-        const int bx = brick / (g.nb[2] * g.nb[1]);
-        // staged region: world texels o + r, r in [0, S), o = b*B - 2
-        const int ox = bx * B - 2, oy = by * B - 2, oz = bz * B - 2;
-        for (int i = threadIdx.x; i < S3; i += kLayoutThreads) {
-            const int rz = i % S, ry = (i / S) % S, rx = i / (S * S);
-            const int x = min(max(ox + rx, 0), g.ext[0] - 1);
-            const int y = min(max(oy + ry, 0), g.ext[1] - 1);
-            const int z = min(max(oz + rz, 0), g.ext[2] - 1);
-            sv[i] = raw_value<T>(vol, z + (long long)g.ext[2] * (y + (long long)g.ext[1] * x));
+build_bricks_kernel(BrickGeometry g, const T *__restrict__ vol, int D, int H, int W, FastDiv by_w, FastDiv by_h,
+                    const float *__restrict__ nrm, Rec *__restrict__ records, uint4 *__restrict__ bricks) {
+    constexpr int B = 1 << LOG2B, A = B + 1, R = A * A * A;
+    const int brick = blockIdx.x;
+    const int bz = brick % g.nb[2], by = (brick / g.nb[2]) % g.nb[1], bx = brick / (g.nb[2] * g.nb[1]);
+    const uint32_t slot = bricks[brick].x;
+    float lo = __int_as_float(0x7f800000), hi = -lo;
+    bool nan = false;
+    for (int rec = threadIdx.x; rec < R; rec += kLayoutThreads) {
+        const int lz = rec % A, ly = (rec / A) % A, lx = rec / (A * A);
+        // record l of the brick holds texel clamp(b*B - 1 + l)
+        const int x = min(max(bx * B - 1 + lx, 0), g.ext[0] - 1);
+        const int y = min(max(by * B - 1 + ly, 0), g.ext[1] - 1);
+        const int z = min(max(bz * B - 1 + lz, 0), g.ext[2] - 1);
+        const uint32_t src = (uint32_t)z + (uint32_t)g.ext[2] * ((uint32_t)y + (uint32_t)g.ext[1] * (uint32_t)x);
+        const float val = raw_value<T>(vol, src);
+        nan |= val != val;
+        lo = fminf(lo, val);
+        hi = fmaxf(hi, val);
+        float3 n;
+        if (nrm) {
+            n = make_float3(nrm[3 * (size_t)src + 0], nrm[3 * (size_t)src + 1], nrm[3 * (size_t)src + 2]);
+        } else {
+            // array position (a, b, c) of flat element src in the (D,H,W) array
+            const uint32_t ab = by_w.quot(src), a = by_h.quot(ab);
+            const int c = (int)(src - ab * by_w.d), b = (int)(ab - a * by_h.d);
+            const uint32_t sa = (uint32_t)H * (uint32_t)W;
+            const float am = (int)a > 0 ? raw_value<T>(vol, src - sa) : 0.0f;
+            const float ap = (int)a < D - 1 ? raw_value<T>(vol, src + sa) : 0.0f;
+            const float bm = b > 0 ? raw_value<T>(vol, src - W) : 0.0f, bp = b < H - 1 ? raw_value<T>(vol, src + W) : 0.0f;
+            const float cm = c > 0 ? raw_value<T>(vol, src - 1) : 0.0f, cp = c < W - 1 ? raw_value<T>(vol, src + 1) : 0.0f;
+            n = GradientArith<T>::finish(GradientArith<T>::axis(am, val, ap, (int)a, D),
+                                         GradientArith<T>::axis(bm, val, bp, b, H),
+                                         GradientArith<T>::axis(cm, val, cp, c, W));
         }
-        __syncthreads();
-        const uint32_t slot = table[brick];
-        float lo = __int_as_float(0x7f800000), hi = -lo;
-        bool nan = false;
-        for (int rec = threadIdx.x; rec < R; rec += kLayoutThreads) {
-            const int lz = rec % A, ly = (rec / A) % A, lx = rec / (A * A);
-            // record l of the brick holds texel clamp(b*B - 1 + l)
-            const int x = min(max(bx * B - 1 + lx, 0), g.ext[0] - 1);
-            const int y = min(max(by * B - 1 + ly, 0), g.ext[1] - 1);
-            const int z = min(max(bz * B - 1 + lz, 0), g.ext[2] - 1);
-            const int ri = ((x - ox) * S + (y - oy)) * S + (z - oz);  // in [1, S-2] per axis
-            const float val = sv[ri];
-            nan |= val != val;
-            lo = fminf(lo, val);
-            hi = fmaxf(hi, val);
-            float3 n = make_float3(0.0f, 0.0f, 0.0f);
-            const long long src = z + (long long)g.ext[2] * (y + (long long)g.ext[1] * x);
-            if (normals_mode == PVR_NORMALS_GIVEN) {
-                n = make_float3(nrm[3 * src + 0], nrm[3 * src + 1], nrm[3 * src + 2]);
-            } else if (normals_mode == PVR_NORMALS_DEVICE) {
-                if (cubic) {
-                    // array position (a, b, c) = (x, y, z)
-                    n = GradientArith<T>::finish(
-                        GradientArith<T>::axis(sv[ri - S * S], val, sv[ri + S * S], x, g.ext[0]),
-                        GradientArith<T>::axis(sv[ri - S], val, sv[ri + S], y, g.ext[1]),
-                        GradientArith<T>::axis(sv[ri - 1], val, sv[ri + 1], z, g.ext[2]));
-                } else {
-                    // array position of flat element `src` in the (D,H,W) array
-                    const int c = (int)(src % W);
-                    const int b = (int)((src / W) % H);
-                    const int a = (int)(src / ((long long)W * H));
-                    n = normal_global<T>(vol, dims, a, b, c);
-                }
-            }
-            records[(size_t)slot * R + rec] = make_record<Rec>(val, n);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        nan = __any_sync(0xffffffffu, nan);
-        if (lane == 0) {
-            s_lo[warp] = lo;
-            s_hi[warp] = hi;
-            s_nan[warp] = nan;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            bool any_nan = false;
-            for (int w = 0; w < WARPS; ++w) {
-                lo = fminf(lo, s_lo[w]);
-                hi = fmaxf(hi, s_hi[w]);
-                any_nan |= s_nan[w] != 0;
-            }
-            bricks[brick] = any_nan ? make_uint4(slot, 0x7fc00000u, 0u, 0u)
-                                    : make_uint4(slot, __float_as_uint(lo), __float_as_uint(hi), 0u);
-        }
-        __syncthreads();  // sv and the partials are rewritten for the next brick
+        records[(size_t)slot * R + rec] = make_record<Rec>(val, n);
     }
+    write_range<kLayoutThreads>(lo, nan ? __int_as_float(0x7fc00000) : hi, bricks + brick);
 }
 
 // A float survives float -> half -> float bit for bit (NaN: as some NaN).
@@ -219,7 +471,7 @@ __device__ __forceinline__ float4 record_at(const uint2 *r, size_t i) {
 // texel, reading the record of local index (k+1) % B in brick (k+1) / B.
 template <int LOG2B, typename Rec>
 __global__ void read_normals_kernel(BrickGeometry g, int D, int H, int W,
-                                    const uint32_t *__restrict__ table,
+                                    const uint4 *__restrict__ bricks,
                                     const Rec *__restrict__ records, float *__restrict__ out) {
     constexpr int B = 1 << LOG2B, A = B + 1, R = A * A * A;
     const long long total = (long long)D * H * W;
@@ -232,51 +484,48 @@ __global__ void read_normals_kernel(BrickGeometry g, int D, int H, int W,
         const int kx = x + 1, ky = y + 1, kz = z + 1;
         const int id = ((kx >> LOG2B) * g.nb[1] + (ky >> LOG2B)) * g.nb[2] + (kz >> LOG2B);
         const int rec = ((kx & (B - 1)) * A + (ky & (B - 1))) * A + (kz & (B - 1));
-        const float4 v = record_at(records, (size_t)table[id] * R + rec);
+        const float4 v = record_at(records, (size_t)bricks[id].x * R + rec);
         out[3 * src + 0] = v.y;
         out[3 * src + 1] = v.z;
         out[3 * src + 2] = v.w;
     }
 }
 
-uint32_t spread3(uint32_t v) {  // 10 bits -> every third bit
-    v &= 0x3ff;
-    v = (v | (v << 16)) & 0x030000ff;
-    v = (v | (v << 8)) & 0x0300f00f;
-    v = (v | (v << 4)) & 0x030c30c3;
-    v = (v | (v << 2)) & 0x09249249;
-    return v;
-}
-
-template <typename T, int LOG2B>
+template <typename T, int LOG2B, typename Rec>
 cudaError_t build_typed(const BrickGeometry &g, const void *vol, const int dims[3], const float *nrm,
-                        int normals_mode, const uint32_t *table, void *records, bool half, uint4 *bricks,
-                        cudaStream_t st) {
+                        int normals_mode, int brick0, int nbricks, Rec *records, uint4 *bricks, cudaStream_t st) {
     // one block per brick: short blocks, so that render kernels on streams
     // of higher priority get SMs as soon as any layout block retires
-    const int blocks = std::max(1, g.nbricks);
-    if (half)
-        build_bricks_kernel<T, LOG2B, uint2><<<blocks, kLayoutThreads, 0, st>>>(
-            g, (const T *)vol, dims[0], dims[1], dims[2], nrm, normals_mode, table, (uint2 *)records, bricks);
+    const bool cubic = dims[0] == dims[1] && dims[1] == dims[2];
+    constexpr int threads = BrickShape<LOG2B>::kThreads;
+    const T *v = (const T *)vol;
+    if (normals_mode == PVR_NORMALS_NONE)
+        build_walk_kernel<T, LOG2B, Rec, false><<<nbricks, threads, 0, st>>>(g, v, brick0, records, bricks);
+    else if (normals_mode == PVR_NORMALS_DEVICE && cubic)
+        build_walk_kernel<T, LOG2B, Rec, true><<<nbricks, threads, 0, st>>>(g, v, brick0, records, bricks);
     else
-        build_bricks_kernel<T, LOG2B, float4><<<blocks, kLayoutThreads, 0, st>>>(
-            g, (const T *)vol, dims[0], dims[1], dims[2], nrm, normals_mode, table, (float4 *)records, bricks);
+        build_bricks_kernel<T, LOG2B, Rec><<<nbricks, kLayoutThreads, 0, st>>>(
+            g, v, dims[0], dims[1], dims[2], FastDiv(dims[2]), FastDiv(dims[1]),
+            normals_mode == PVR_NORMALS_GIVEN ? nrm : nullptr, records, bricks);
     return cudaGetLastError();
 }
 
 template <int LOG2B>
 cudaError_t build_log2(const BrickGeometry &g, int dtype, const void *vol, const int dims[3],
-                       const float *nrm, int normals_mode, const uint32_t *table, void *records, bool half,
+                       const float *nrm, int normals_mode, int brick0, int nbricks, void *records, bool half,
                        uint4 *bricks, cudaStream_t st) {
-    switch (dtype) {
-    case PVR_U8:
-        return build_typed<uint8_t, LOG2B>(g, vol, dims, nrm, normals_mode, table, records, half, bricks, st);
-    case PVR_F16:
-        return build_typed<__half, LOG2B>(g, vol, dims, nrm, normals_mode, table, records, half, bricks, st);
-    default:
-        // float32 values are not halves: float records only
-        return build_typed<float, LOG2B>(g, vol, dims, nrm, normals_mode, table, records, false, bricks, st);
-    }
+    if (dtype == PVR_F32)  // float32 values are not halves: float records only
+        return build_typed<float, LOG2B, float4>(g, vol, dims, nrm, normals_mode, brick0, nbricks, (float4 *)records,
+                                                 bricks, st);
+    if (dtype == PVR_U8)
+        return half ? build_typed<uint8_t, LOG2B, uint2>(g, vol, dims, nrm, normals_mode, brick0, nbricks,
+                                                         (uint2 *)records, bricks, st)
+                    : build_typed<uint8_t, LOG2B, float4>(g, vol, dims, nrm, normals_mode, brick0, nbricks,
+                                                          (float4 *)records, bricks, st);
+    return half ? build_typed<__half, LOG2B, uint2>(g, vol, dims, nrm, normals_mode, brick0, nbricks,
+                                                    (uint2 *)records, bricks, st)
+                : build_typed<__half, LOG2B, float4>(g, vol, dims, nrm, normals_mode, brick0, nbricks,
+                                                     (float4 *)records, bricks, st);
 }
 
 }  // namespace
@@ -293,49 +542,42 @@ BrickGeometry make_brick_geometry(const int dims_dhw[3], int log2b) {
     return g;
 }
 
-// Slot of every brick: rank of its Morton code (x, y, z interleaved).
-std::vector<uint32_t> morton_slots(const BrickGeometry &g) {
-    std::vector<std::pair<uint64_t, uint32_t>> key(g.nbricks);
-    for (int bx = 0; bx < g.nb[0]; ++bx)
-        for (int by = 0; by < g.nb[1]; ++by)
-            for (int bz = 0; bz < g.nb[2]; ++bz) {
-                uint32_t id = (uint32_t)((bx * g.nb[1] + by) * g.nb[2] + bz);
-                uint64_t m = ((uint64_t)spread3(bx) << 2) | ((uint64_t)spread3(by) << 1) | spread3(bz);
-                key[id] = {m, id};
-            }
-    std::sort(key.begin(), key.end());
-    std::vector<uint32_t> table(g.nbricks);
-    for (uint32_t s = 0; s < (uint32_t)g.nbricks; ++s) table[key[s].second] = s;
-    return table;
+cudaError_t launch_brick_slots(const BrickGeometry &g, uint4 *bricks, cudaStream_t st) {
+    brick_slots_kernel<<<(g.nbricks + 127) / 128, 128, 0, st>>>(g, bricks);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_build_records(const BrickGeometry &g, int dtype, const void *vol, const int dims[3],
-                                 const float *nrm, int normals_mode, const uint32_t *table,
-                                 void *records, bool half, uint4 *bricks, cudaStream_t st) {
+                                 const float *nrm, int normals_mode, int brick0, int nbricks, void *records, bool half,
+                                 uint4 *bricks, cudaStream_t st) {
     if (half && dtype == PVR_F32) return cudaErrorInvalidValue;
+    if (nbricks <= 0) return cudaSuccess;
     switch (g.log2b) {
-    case 2: return build_log2<2>(g, dtype, vol, dims, nrm, normals_mode, table, records, half, bricks, st);
-    case 4: return build_log2<4>(g, dtype, vol, dims, nrm, normals_mode, table, records, half, bricks, st);
-    default: return build_log2<3>(g, dtype, vol, dims, nrm, normals_mode, table, records, half, bricks, st);
+    case 2:
+        return build_log2<2>(g, dtype, vol, dims, nrm, normals_mode, brick0, nbricks, records, half, bricks, st);
+    case 4:
+        return build_log2<4>(g, dtype, vol, dims, nrm, normals_mode, brick0, nbricks, records, half, bricks, st);
+    default:
+        return build_log2<3>(g, dtype, vol, dims, nrm, normals_mode, brick0, nbricks, records, half, bricks, st);
     }
 }
 
 template <typename Rec>
-void read_normals_typed(const BrickGeometry &g, const int dims[3], const uint32_t *table, const Rec *records,
+void read_normals_typed(const BrickGeometry &g, const int dims[3], const uint4 *bricks, const Rec *records,
                         float *out, int blocks, cudaStream_t st) {
     switch (g.log2b) {
-    case 2: read_normals_kernel<2><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], table, records, out); break;
-    case 4: read_normals_kernel<4><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], table, records, out); break;
-    default: read_normals_kernel<3><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], table, records, out);
+    case 2: read_normals_kernel<2><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], bricks, records, out); break;
+    case 4: read_normals_kernel<4><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], bricks, records, out); break;
+    default: read_normals_kernel<3><<<blocks, 256, 0, st>>>(g, dims[0], dims[1], dims[2], bricks, records, out);
     }
 }
 
-cudaError_t launch_read_normals(const BrickGeometry &g, const int dims[3], const uint32_t *table,
+cudaError_t launch_read_normals(const BrickGeometry &g, const int dims[3], const uint4 *bricks,
                                 const void *records, bool compact, float *out, cudaStream_t st) {
     const long long total = (long long)dims[0] * dims[1] * dims[2];
     int blocks = (int)std::min<long long>((total + 255) / 256, 152LL * 64);
-    if (compact) read_normals_typed(g, dims, table, (const uint2 *)records, out, blocks, st);
-    else read_normals_typed(g, dims, table, (const float4 *)records, out, blocks, st);
+    if (compact) read_normals_typed(g, dims, bricks, (const uint2 *)records, out, blocks, st);
+    else read_normals_typed(g, dims, bricks, (const float4 *)records, out, blocks, st);
     return cudaGetLastError();
 }
 

@@ -35,17 +35,20 @@ struct BrickGeometry {
 };
 
 BrickGeometry make_brick_geometry(const int dims_dhw[3], int log2b);
-std::vector<uint32_t> morton_slots(const BrickGeometry &g);
 
 // normals_mode: 0 none, 1 from `nrm` (float32 (D,H,W,3)), 2 computed on the
 // device from the stored values (numpy.gradient semantics).
 // bricks[b] = {record slot, min, max (float bits), 0}: what the march needs
 // when a ray enters brick b, in one 16-byte load.
 // half: 8-byte half records (uint8 / float16 volumes only).
+// launch_brick_slots writes the slots; launch_build_records then the records
+// and value ranges of bricks [brick0, brick0 + nbricks) (x-major order).
+// Device normals of non-cubic volumes and given normals: all bricks at once.
+cudaError_t launch_brick_slots(const BrickGeometry &g, uint4 *bricks, cudaStream_t st);
 cudaError_t launch_build_records(const BrickGeometry &g, int dtype, const void *vol, const int dims[3],
-                                 const float *nrm, int normals_mode, const uint32_t *table,
-                                 void *records, bool half, uint4 *bricks, cudaStream_t st);
-cudaError_t launch_read_normals(const BrickGeometry &g, const int dims[3], const uint32_t *table,
+                                 const float *nrm, int normals_mode, int brick0, int nbricks, void *records,
+                                 bool half, uint4 *bricks, cudaStream_t st);
+cudaError_t launch_read_normals(const BrickGeometry &g, const int dims[3], const uint4 *bricks,
                                 const void *records, bool compact, float *out, cudaStream_t st);
 // Half-precision copy of n records ({value, nx, ny, nz} as four halves, 8
 // bytes); *inexact is set to 1 if some float does not survive the round trip
@@ -144,7 +147,6 @@ struct pvr_volume {
     size_t records_bytes = 0;
     bool compact = false;       // records stored as halves
     bool compact_exact = true;  // ... and every float of them survived exactly
-    uint32_t *d_table = nullptr;  // brick -> record slot
     uint4 *d_bricks = nullptr;    // brick -> {slot, min, max}
     bool layout_ready = false;    // the layout is built or queued
     // recorded after the layout's work (volumes created by pvr_volume_create*):

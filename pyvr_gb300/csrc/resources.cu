@@ -107,11 +107,9 @@ void free_volume_buffers(pvr_volume *v, cudaStream_t st) {
     vol_free(v->d_vol, st);
     vol_free(v->d_nrm, st);
     vol_free(v->d_records, st);
-    vol_free(v->d_table, st);
     vol_free(v->d_bricks, st);
     v->d_vol = v->d_nrm = nullptr;
     v->d_records = nullptr;
-    v->d_table = nullptr;
     v->d_bricks = nullptr;
 }
 
@@ -127,19 +125,14 @@ static std::atomic<int> g_arithmetic{PVR_ARITH_FAST};
 
 bool arithmetic_fast() { return g_arithmetic.load(std::memory_order_relaxed) == PVR_ARITH_FAST; }
 
-// The allocations of a volume's layout and the upload of its brick table
-// (from pageable memory: on a stream with no work queued yet, the copy is
-// staged and returns at once).
+// The allocations of a volume's layout, and its brick slots.
 static int layout_prepare(pvr_volume *v, cudaStream_t st, bool &half) {
     vol_free(v->d_records, st);
-    vol_free(v->d_table, st);
     vol_free(v->d_bricks, st);
     v->d_records = nullptr;
-    v->d_table = nullptr;
     v->d_bricks = nullptr;
     v->records_bytes = 0;
     v->geo = make_brick_geometry(v->dims, v->log2b);
-    std::vector<uint32_t> table = morton_slots(v->geo);
     const size_t nrec = (size_t)v->geo.nbricks * brick_records(v->log2b);
     // half records written directly: values of uint8 / float16 volumes are
     // halves exactly; normals are rounded to half
@@ -147,18 +140,15 @@ static int layout_prepare(pvr_volume *v, cudaStream_t st, bool &half) {
     const size_t rec_size = half ? sizeof(uint2) : sizeof(float4);
     PVR_CUDA(vol_alloc((void **)&v->d_records, nrec * rec_size, st));
     v->records_bytes = nrec * rec_size;
-    PVR_CUDA(vol_alloc((void **)&v->d_table, table.size() * sizeof(uint32_t), st));
-    PVR_CUDA(vol_alloc((void **)&v->d_bricks, table.size() * sizeof(uint4), st));
-    // pageable source: staged before the call returns, so `table` may go
-    PVR_CUDA(cudaMemcpyAsync(v->d_table, table.data(), table.size() * sizeof(uint32_t),
-                             cudaMemcpyHostToDevice, st));
+    PVR_CUDA(vol_alloc((void **)&v->d_bricks, (size_t)v->geo.nbricks * sizeof(uint4), st));
+    PVR_CUDA(launch_brick_slots(v->geo, v->d_bricks, st));
     return PVR_OK;
 }
 
 // The layout kernel over the uploaded voxels (and given normals).
 static int layout_launch(pvr_volume *v, cudaStream_t st, bool half) {
-    PVR_CUDA(launch_build_records(v->geo, v->dtype, v->d_vol, v->dims, v->d_nrm, v->normals_mode,
-                                  v->d_table, v->d_records, half, v->d_bricks, st));
+    PVR_CUDA(launch_build_records(v->geo, v->dtype, v->d_vol, v->dims, v->d_nrm, v->normals_mode, 0,
+                                  v->geo.nbricks, v->d_records, half, v->d_bricks, st));
     vol_free(v->d_nrm, st);  // given normals now live in the records
     v->d_nrm = nullptr;
     v->compact = half;
@@ -356,8 +346,7 @@ static int create_volume(const void *data, int dtype, int d, int h, int w, float
         delete v;
         return rc;
     };
-    // the brick table first, while the stream is empty (its pageable copy
-    // then returns at once), then the voxels in their storage type
+    // the brick slots, then the voxels in their storage type
     bool half = false;
     if (int rc = pvr::layout_prepare(v, st, half)) return bail(rc);
     e = pvr::vol_alloc(&v->d_vol, nvox * dtype_size(dtype), st);
@@ -549,7 +538,7 @@ int pvr_volume_records_exact(const pvr_volume *v, int *exact) {
 int pvr_volume_device_bytes(const pvr_volume *v, long long *bytes) {
     if (!v || !bytes) return fail(PVR_ERR_VALUE, "NULL argument");
     *bytes = (long long)(v->vol_bytes + v->records_bytes +
-                         (size_t)v->geo.nbricks * (sizeof(uint32_t) + sizeof(uint4)));
+                         (size_t)v->geo.nbricks * sizeof(uint4));
     return PVR_OK;
 }
 
@@ -560,7 +549,7 @@ int pvr_volume_read_normals(const pvr_volume *v, float *normals_out) {
     const size_t n = (size_t)v->dims[0] * v->dims[1] * v->dims[2] * 3;
     float *d = nullptr;
     PVR_CUDA(cudaMalloc(&d, n * sizeof(float)));
-    cudaError_t e = pvr::launch_read_normals(v->geo, v->dims, v->d_table, v->d_records, v->compact, d, 0);
+    cudaError_t e = pvr::launch_read_normals(v->geo, v->dims, v->d_bricks, v->d_records, v->compact, d, 0);
     if (e == cudaSuccess) e = cudaMemcpy(normals_out, d, n * sizeof(float), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return pvr::cuda_fail(e, "read normals");
