@@ -2,6 +2,7 @@
 // pyvr/moderngl_renderer/manager.py:77-135 as bricked texel records) and
 // RGBA LUTs (manager.py:137-186), plus the host-side derivations shared by
 // the renderer and the batch launcher.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
@@ -145,10 +146,61 @@ static int layout_prepare(pvr_volume *v, cudaStream_t st, bool &half) {
     return PVR_OK;
 }
 
-// The layout kernel over the uploaded voxels (and given normals).
-static int layout_launch(pvr_volume *v, cudaStream_t st, bool half) {
-    PVR_CUDA(launch_build_records(v->geo, v->dtype, v->d_vol, v->dims, v->d_nrm, v->normals_mode, 0,
-                                  v->geo.nbricks, v->d_records, half, v->d_bricks, st));
+// The layout kernel over the uploaded voxels (and given normals): bricks
+// [bx0, bx1) along world x.
+static int layout_bricks(pvr_volume *v, cudaStream_t st, bool half, int bx0, int bx1) {
+    const int per_x = v->geo.nb[1] * v->geo.nb[2];
+    PVR_CUDA(launch_build_records(v->geo, v->dtype, v->d_vol, v->dims, v->d_nrm, v->normals_mode, bx0 * per_x,
+                                  (bx1 - bx0) * per_x, v->d_records, half, v->d_bricks, st));
+    return PVR_OK;
+}
+
+// Uploads the voxels in slabs along world x (the slowest axis of the buffer)
+// on a stream of their own, and lays out the bricks of a slab on `st` as soon
+// as the texels they and their normals read have arrived, while the next
+// slab is on its way: a large volume is ready shortly after its last byte
+// (512^3 float16 from page-locked memory: upload 1.29 ms, then layout 0.56 ms:
+// 1.93 -> 1.50 ms; uint8 1.18 -> 0.84 ms).  Slabs of 16 MB and more, at most 8: a slab's copy
+// (80 us) then outweighs its launch, and the last slab's layout, which
+// nothing hides, stays an eighth of the whole.
+static int upload_and_layout(pvr_volume *v, const char *data, cudaStream_t st, bool half) {
+    const int ext = v->geo.ext[0], B = 1 << v->log2b;
+    const size_t per_x = v->vol_bytes / (size_t)ext;
+    const int slabs = (int)std::min<size_t>(8, v->vol_bytes >> 24);
+    cudaStream_t up = nullptr;
+    cudaEvent_t arrived = nullptr;
+    int lo = 0, hi = 0;
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    cudaError_t e = cudaStreamCreateWithPriority(&up, cudaStreamNonBlocking, hi);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&arrived, cudaEventDisableTiming);
+    // the buffer was allocated in the order of `st`
+    if (e == cudaSuccess) e = cudaEventRecord(arrived, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(up, arrived, 0);
+    int rc = PVR_OK, x0 = 0, b0 = 0;
+    for (int i = 1; i <= slabs && e == cudaSuccess && rc == PVR_OK; ++i) {
+        // brick b reads texels up to (b + 1) * B (its apron's neighbour)
+        const int b1 = i == slabs ? v->geo.nb[0] : (int)((long long)v->geo.nb[0] * i / slabs);
+        const int x1 = i == slabs ? ext : std::min(ext, b1 * B + 1);
+        if (x1 > x0)
+            e = cudaMemcpyAsync((char *)v->d_vol + x0 * per_x, data + x0 * per_x, (size_t)(x1 - x0) * per_x,
+                                cudaMemcpyHostToDevice, up);
+        if (e == cudaSuccess) e = cudaEventRecord(arrived, up);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, arrived, 0);
+        if (e == cudaSuccess) rc = layout_bricks(v, st, half, b0, b1);
+        x0 = std::max(x0, x1);
+        b0 = b1;
+    }
+    if (e != cudaSuccess || rc != PVR_OK) {
+        if (up) cudaStreamSynchronize(up);  // the caller frees the buffer
+        if (rc == PVR_OK) rc = cuda_fail(e, "upload volume");
+    }
+    if (arrived) cudaEventDestroy(arrived);
+    if (up) cudaStreamDestroy(up);  // its queued copies still run
+    return rc;
+}
+
+// What follows the layout's kernels.
+static void layout_queued(pvr_volume *v, cudaStream_t st, bool half) {
     vol_free(v->d_nrm, st);  // given normals now live in the records
     v->d_nrm = nullptr;
     v->compact = half;
@@ -156,7 +208,6 @@ static int layout_launch(pvr_volume *v, cudaStream_t st, bool half) {
     // precision (numpy's arithmetic for float16 input)
     v->compact_exact = !half || v->normals_mode == PVR_NORMALS_NONE ||
                        (v->dtype == PVR_F16 && v->normals_mode == PVR_NORMALS_DEVICE);
-    return PVR_OK;
 }
 
 // Records, brick table and value ranges of a volume (once per volume).
@@ -164,7 +215,8 @@ int ensure_volume_layout(pvr_volume *v, cudaStream_t st) {
     if (v->layout_ready) return PVR_OK;
     bool half = false;
     if (int rc = layout_prepare(v, st, half)) return rc;
-    if (int rc = layout_launch(v, st, half)) return rc;
+    if (int rc = layout_bricks(v, st, half, 0, v->geo.nb[0])) return rc;
+    layout_queued(v, st, half);
     PVR_CUDA(cudaStreamSynchronize(st));  // ready for any stream
     v->layout_ready = true;
     if (g_compact_records.load() == PVR_RECORDS_HALF_EXACT) try_compact_records(v, st, false);
@@ -352,15 +404,24 @@ static int create_volume(const void *data, int dtype, int d, int h, int w, float
     e = pvr::vol_alloc(&v->d_vol, nvox * dtype_size(dtype), st);
     if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "allocate volume"));
     v->vol_bytes = nvox * dtype_size(dtype);
-    e = cudaMemcpyAsync(v->d_vol, data, v->vol_bytes, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "upload volume"));
-    if (normals_mode == PVR_NORMALS_GIVEN) {
-        e = pvr::vol_alloc((void **)&v->d_nrm, nvox * 3 * sizeof(float), st);
-        if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "allocate normals"));
-        e = cudaMemcpyAsync(v->d_nrm, normals, nvox * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "upload normals"));
+    // in slabs where the bricks of a slab depend on nothing beyond it: not
+    // with device normals of a non-cubic volume (its array neighbours are not
+    // world neighbours), nor with given normals (three more uploads)
+    if (v->vol_bytes >= (32u << 20) &&
+        (normals_mode == PVR_NORMALS_NONE || (normals_mode == PVR_NORMALS_DEVICE && d == h && h == w))) {
+        if (int rc = pvr::upload_and_layout(v, static_cast<const char *>(data), st, half)) return bail(rc);
+    } else {
+        e = cudaMemcpyAsync(v->d_vol, data, v->vol_bytes, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "upload volume"));
+        if (normals_mode == PVR_NORMALS_GIVEN) {
+            e = pvr::vol_alloc((void **)&v->d_nrm, nvox * 3 * sizeof(float), st);
+            if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "allocate normals"));
+            e = cudaMemcpyAsync(v->d_nrm, normals, nvox * 3 * sizeof(float), cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) return bail(pvr::cuda_fail(e, "upload normals"));
+        }
+        if (int rc = pvr::layout_bricks(v, st, half, 0, v->geo.nb[0])) return bail(rc);
     }
-    if (int rc = pvr::layout_launch(v, st, half)) return bail(rc);
+    pvr::layout_queued(v, st, half);
     // the records hold every stored value: the uploaded voxels are not needed
     // again (a volume resource is never laid out twice)
     pvr::vol_free(v->d_vol, st);

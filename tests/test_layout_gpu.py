@@ -96,3 +96,41 @@ def test_half_normals_exhaustive(tmp_path):
     assert u8_bad == 0, f"{u8_bad} of {triples} uint8 components differ"
     assert undecided < 0.01 * triples, undecided
     assert f16_bad == 0, f"{f16_bad} of {pairs} float16 quotients differ"
+
+
+@pytest.mark.parametrize("dims,dtype,normals,brick", [((257,) * 3, "f16", "device", 3), ((262,) * 3, "f16", "device", 4),
+                                                      ((300, 41, 700), "f32", "none", 3), ((3000, 4000, 3), "u8", "none", 4)])
+def test_upload_in_slabs(dims, dtype, normals, brick):
+    # 32 MB and more arrive in slabs, each laid out while the next is copied:
+    # normals and frames as for a volume that arrived whole
+    from pyvr_gb300.batch import (BatchRenderer, DeviceLUT, DeviceVolume, RenderJob, arithmetic,
+                                  get_compact_records, page_locked_copy, set_compact_records)
+    from pyvr_gb300.renderer import rgba_lut
+    data = page_locked_copy(_data(dims, dtype, 77))
+    with np.errstate(all="ignore"):
+        nrm = compute_normal_volume(data) if normals == "device" else None
+    vol = Volume(data=data, min_bounds=np.full(3, -1.0, np.float32), max_bounds=np.full(3, 1.0, np.float32))
+    prev = get_compact_records()
+    set_compact_records("half_normals")
+    try:
+        dv = DeviceVolume(vol, normals=normals, brick_log2=brick, wait=False)
+    finally:
+        set_compact_records(prev)
+    cam, light, cfg = W.config_small()["camera"], W.config_small()["light"], RenderConfig.fast()
+    ctf, otf = W.standin_colormap(2), W.random_opacity(np.random.default_rng(5), 6, 0.3)
+    w, h = 61, 52
+    outf = torch.empty(w * h * 4, dtype=torch.float32, device="cuda")
+    br = BatchRenderer(capacity=1, slots=1)
+    with arithmetic("exact"):
+        br.render([RenderJob(dv, DeviceLUT(ctf, otf), cam, light, cfg, w, h, None, outf)])
+        br.synchronize()
+    if nrm is not None:
+        assert np.array_equal(dv.read_normals(), nrm.astype(np.float32), equal_nan=True)
+        vol.normals = nrm.astype(np.float32)
+    _, of, _ = oracle.render(W.frame_inputs(vol, cam, light, cfg, rgba_lut(ctf, otf), w, h, 1.0, batch_camera=True))
+    got = outf.cpu().numpy().reshape(h, w, 4)
+    finite = np.isfinite(of).all(axis=2)
+    assert np.array_equal(got[finite].view(np.uint32), of[finite].view(np.uint32))
+    assert np.array_equal(np.isfinite(got).all(axis=2), finite)
+    br.close()
+    dv.close()
