@@ -127,7 +127,8 @@ def _march_function():
             ws = _workspace(n.value, volume.device)
             check(_lib().pvr_diff_forward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), ws[1], ws[2],
                                              stream))
-            ctx.scene = scene
+            # the scene as it was rendered; the backward puts its own tensors' addresses in
+            ctx.scene, ctx.c = scene, c
             ctx.workspace_bytes = (n.value, n_vol.value)
             ctx.save_for_backward(volume, lut, normals, image, steps)
             ctx.mark_non_differentiable(steps)
@@ -141,7 +142,9 @@ def _march_function():
             glut = torch.zeros_like(lut) if need_lut else None
             if need_vol or need_lut:
                 gimage = gimage.contiguous()
-                c = ctx.scene.c_scene(volume, lut, normals)
+                c = ctx.c
+                c.volume, c.lut = volume.data_ptr(), lut.data_ptr()
+                c.normals = normals.data_ptr() if normals is not None else None
                 stream = torch.cuda.current_stream(volume.device).cuda_stream
                 ws = _workspace(ctx.workspace_bytes[1 if need_vol else 0], volume.device)
                 check(_lib().pvr_diff_backward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(),
