@@ -28,6 +28,11 @@ def _cases():
         (W.standin_colormap(4), W.random_opacity(rng, 8, 0.3), 1),
         (W.standin_colormap(5), W.random_opacity(rng, 8, 0.3), 2),
         (W.standin_colormap(6), W.random_opacity(rng, 8, 0.3), 65536),
+        # on both sides of the small parameter block, and the largest
+        (W.standin_colormap(7), W.random_opacity(rng, 32, 0.3), 33),
+        (W.standin_colormap(8), W.random_opacity(rng, 33, 0.3), 1025),
+        (CTF([(float(x), tuple(rng.random(3).tolist())) for x in np.sort(rng.random(256))]),
+         W.random_opacity(rng, 256, 0.3), 640),
     ]
     return out
 
