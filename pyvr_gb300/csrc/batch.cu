@@ -23,6 +23,9 @@ const void *batch_kernel_b4(const Tuning &, int);
 const void *single_kernel_b2(const Tuning &, int);
 const void *single_kernel_b3(const Tuning &, int);
 const void *single_kernel_b4(const Tuning &, int);
+const void *split_kernel_b2(int, int);
+const void *split_kernel_b3(int, int);
+const void *split_kernel_b4(int, int);
 int max_batch_blocks_b2(const Tuning &, int, int);
 int max_batch_blocks_b3(const Tuning &, int, int);
 int max_batch_blocks_b4(const Tuning &, int, int);
@@ -40,6 +43,14 @@ const void *single_kernel(int log2b, const Tuning &t, int variant) {
     case 2: return single_kernel_b2(t, variant);
     case 4: return single_kernel_b4(t, variant);
     default: return single_kernel_b3(t, variant);
+    }
+}
+
+const void *split_kernel(int log2b, int lanes, int variant) {
+    switch (log2b) {
+    case 2: return split_kernel_b2(lanes, variant);
+    case 4: return split_kernel_b4(lanes, variant);
+    default: return split_kernel_b3(lanes, variant);
     }
 }
 
@@ -92,6 +103,7 @@ struct pvr_batch {
     std::vector<Slot> slots;
     std::unique_ptr<pvr::BatchParams> params;  // host staging of one launch's job table
     pvr::SingleParams single;                  // ... of a one-job launch
+    bool split = true;  // small single renders may take several lanes per ray
 };
 
 using pvr::fail;
@@ -157,6 +169,19 @@ int build_graph(Slot &s, const LaunchKey &key, void **args) {
     return PVR_OK;
 }
 
+// Lanes per ray of a single render that has the chip to itself, by its pixels
+// per SM.  Device us with 1 / 2 / 4 lanes, 256^3 uint8 in float records and
+// 384^3 float16 in half records (balanced), 64^3 float32 (high quality):
+//   192^2   59.8 / 40.2 / 38.7    79.5 / 41.1 / 34.9    63.6 / 44.2 / 36.8
+//   256^2   64.3 / 55.1 / 59.1    84.0 / 53.7 / 52.4    65.0 / 57.7 / 53.5
+//   384^2   78.5 / 78.2 / 87.5    93.9 / 83.1 / 81.2    87.4 / 85.5 / 89.5
+//   512^2  102.7 / 103.7 / 130   103.5 / 104.5 / 117   122.7 / 125.7 / 142
+constexpr int kSplit4Pixels = 330, kSplit2Pixels = 970;  // 224^2 and 384^2 on 152 SMs
+int split_lanes(int width, int height, int sms) {
+    const long long pixels = (long long)width * height;
+    return pixels <= (long long)kSplit4Pixels * sms ? 4 : pixels <= (long long)kSplit2Pixels * sms ? 2 : 1;
+}
+
 // One launch over jobs[idx[0..n)] (jobs of one variant, at most
 // kMaxLaunchJobs).
 int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool fast, cudaStream_t st) {
@@ -175,7 +200,10 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
         // launched directly (its parameters are copied at the launch, and it
         // uses no work counter); the slot's event tracks it like a batch
         pvr::SingleParams &sp = b->single;
-        if (int rc = pvr::fill_job(jobs[0], b->tuning.tile_w, b->tuning.tile_h, fast, sp.job)) return rc;
+        const int lanes = b->split ? split_lanes(jobs[0].width, jobs[0].height, b->sms) : 1;
+        const int tile_w = lanes > 1 ? pvr::split_tile_w(lanes) : b->tuning.tile_w;
+        const int tile_h = lanes > 1 ? pvr::split_tile_h(lanes) : b->tuning.tile_h;
+        if (int rc = pvr::fill_job(jobs[0], tile_w, tile_h, fast, sp.job)) return rc;
         sp.tile_w = b->tuning.tile_w;
         sp.tile_h = b->tuning.tile_h;
         int lut_smem = 256;
@@ -186,7 +214,8 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
                             (sp.job.compact ? pvr::kSingleCompact : 0) | (fast ? pvr::kSingleFast : 0);
         const long long tiles = (long long)sp.job.tiles_x * sp.job.tiles_y;
         void *args[] = {&sp};
-        PVR_CUDA(cudaLaunchKernel(pvr::single_kernel(log2b, b->tuning, variant), dim3((unsigned)tiles),
+        PVR_CUDA(cudaLaunchKernel(lanes > 1 ? pvr::split_kernel(log2b, lanes, variant)
+                                            : pvr::single_kernel(log2b, b->tuning, variant), dim3((unsigned)tiles),
                                   dim3(pvr::kBatchThreads), args, smem ? pvr::batch_smem_bytes(lut_smem) : 0,
                                   st));
         PVR_CUDA(cudaEventRecord(s.done, st));
@@ -240,6 +269,8 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
 }
 
 }  // namespace
+
+void pvr::batch_allow_split(pvr_batch *b, bool allow) { b->split = allow; }
 
 extern "C" {
 

@@ -93,12 +93,32 @@ __device__ __forceinline__ int lut_index(float fl, float lmax) {
     return (int)fminf(fmaxf(fl, 0.0f), lmax);
 }
 
-// Shading + compositing of one in-box sample (frag:93-115).  p: the record
-// of the footprint's lower corner; fx, fy, fz: the filter fractions.
+// What one sample adds before its transmittance: (r, g) and (b, alpha).
+struct Source {
+    float2 rg, ba;
+};
+
+// Front-to-back compositing (frag:112-115):
+// acc.c += (1 - acc.a) * (c * light * alpha), acc.a += (1 - acc.a) * alpha
+template <bool FAST>
+__device__ __forceinline__ void composite(const Source &s, float2 &acc_rg, float2 &acc_ba) {
+    const float2 tr = dup2(__fadd_rn(1.0f, -acc_ba.y));
+    if (FAST) {
+        acc_rg = __ffma2_rn(tr, s.rg, acc_rg);
+        acc_ba = __ffma2_rn(tr, s.ba, acc_ba);
+        return;
+    }
+    const float2 add_rg = __fmul2_rn(tr, s.rg);
+    const float2 add_ba = __fmul2_rn(tr, s.ba);
+    acc_rg = make_float2(__fadd_rn(acc_rg.x, add_rg.x), __fadd_rn(acc_rg.y, add_rg.y));
+    acc_ba = make_float2(__fadd_rn(acc_ba.x, add_ba.x), __fadd_rn(acc_ba.y, add_ba.y));
+}
+
+// Shading of one in-box sample (frag:93-110).  p: the record of the
+// footprint's lower corner; fx, fy, fz: the filter fractions.
 template <int LOG2B, bool NORMALS, bool SMEM_LUT, bool FAST, typename Rec>
-__device__ __forceinline__ void shade_sample(const MarchFrame &f, const Rec *__restrict__ p,
-                                             float fx, float fy, float fz, const float4 *lut,
-                                             float2 &acc_rg, float2 &acc_ba) {
+__device__ __forceinline__ Source shade_sample(const MarchFrame &f, const Rec *__restrict__ p,
+                                               float fx, float fy, float fz, const float4 *lut) {
     constexpr int ROW = brick_apron(LOG2B), SLICE = ROW * ROW;
     float density;
     float n[3];
@@ -171,11 +191,7 @@ __device__ __forceinline__ void shade_sample(const MarchFrame &f, const Rec *__r
         const float dl = fmaf(n[0], f.light_dir[0], fmaf(n[1], f.light_dir[1], __fmul_rn(n[2], f.light_dir[2])));
         const float di = n2 > 0.0f ? fmaxf(__fmul_rn(dl, rsqrt_approx(n2)), 0.0f) : 0.0f;
         const float la_ = __fmul_rn(fmaf(f.diffuse, di, f.ambient), alpha);
-        // front-to-back compositing (frag:112-115)
-        const float2 tr = dup2(__fadd_rn(1.0f, -acc_ba.y));
-        acc_rg = __ffma2_rn(tr, __fmul2_rn(crg, dup2(la_)), acc_rg);
-        acc_ba = __ffma2_rn(tr, make_float2(__fmul_rn(cba.x, la_), alpha), acc_ba);
-        return;
+        return {__fmul2_rn(crg, dup2(la_)), make_float2(__fmul_rn(cba.x, la_), alpha)};
     }
 
     // Beer-Lambert opacity correction (frag:101)
@@ -194,15 +210,8 @@ __device__ __forceinline__ void shade_sample(const MarchFrame &f, const Rec *__r
         di = fmaxf(d, 0.0f);
     }
     const float light = __fadd_rn(f.ambient, __fmul_rn(f.diffuse, di));
-    // front-to-back compositing (frag:112-115):
-    // acc.c += (1 - acc.a) * (c * light * alpha), acc.a += (1 - acc.a) * alpha
-    const float2 tr = dup2(__fadd_rn(1.0f, -acc_ba.y));
-    const float2 src_rg = __fmul2_rn(__fmul2_rn(crg, dup2(light)), dup2(alpha));
-    const float src_b = __fmul_rn(__fmul_rn(cba.x, light), alpha);
-    const float2 add_rg = __fmul2_rn(tr, src_rg);
-    const float2 add_ba = __fmul2_rn(tr, make_float2(src_b, alpha));
-    acc_rg = make_float2(__fadd_rn(acc_rg.x, add_rg.x), __fadd_rn(acc_rg.y, add_rg.y));
-    acc_ba = make_float2(__fadd_rn(acc_ba.x, add_ba.x), __fadd_rn(acc_ba.y, add_ba.y));
+    return {__fmul2_rn(__fmul2_rn(crg, dup2(light)), dup2(alpha)),
+            make_float2(__fmul_rn(__fmul_rn(cba.x, light), alpha), alpha)};
 }
 
 __device__ __forceinline__ uint32_t blend_rgba8(float2 rg, float2 ba) {
@@ -289,9 +298,9 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
                 if (!clear) {
                     ++n_shaded;
                     const int j = (kx & (B - 1)) * SLICE + (ky & (B - 1)) * ROW + (kz & (B - 1));
-                    shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST>(f, bp + j, __fadd_rn(ux, -flx),
-                                                                 __fadd_rn(uy, -fly), __fadd_rn(uz, -flz),
-                                                                 lut, acc_rg, acc_ba);
+                    composite<FAST>(shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST>(
+                                        f, bp + j, __fadd_rn(ux, -flx), __fadd_rn(uy, -fly), __fadd_rn(uz, -flz), lut),
+                                    acc_rg, acc_ba);
                 }
             } else {
                 const bool never = entered || (txy.x < 0.0f && dxy.x <= 0.0f) ||
@@ -328,16 +337,11 @@ __device__ __forceinline__ void stage_lut(float4 *s_lut, int *s_prefix, const Jo
     for (int k = threadIdx.x; k <= size; k += kBatchThreads) s_prefix[k] = job.prefix[k];
 }
 
-template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
-__device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, const float4 *lut,
-                                           const int *prefix, int lane) {
-    const bool in_image = px < job.f.width && py < job.f.height;
-    float2 acc_rg = make_float2(0.0f, 0.0f), acc_ba = make_float2(0.0f, 0.0f);
-    unsigned n_inbox = 0, n_shaded = 0;
-    if (in_image)
-        march_ray<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, lut, prefix, acc_rg, acc_ba,
-                                                                   n_inbox, n_shaded);
-    if (in_image) {
+// Writes the lane's pixel (writes: it has one) and adds the warp's sample
+// counts.
+__device__ __forceinline__ void store_pixel(const JobDesc &job, int px, int py, bool writes, float2 acc_rg,
+                                            float2 acc_ba, unsigned n_inbox, unsigned n_shaded, int lane) {
+    if (writes) {
         const long long idx = (long long)py * job.f.width + px;
         if (job.out8) job.out8[idx] = blend_rgba8(acc_rg, acc_ba);
         if (job.outf) job.outf[idx] = make_float4(acc_rg.x, acc_rg.y, acc_ba.x, acc_ba.y);
@@ -354,6 +358,18 @@ __device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, c
             atomicAdd(job.counters + 1, b);
         }
     }
+}
+
+template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
+__device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, const float4 *lut,
+                                           const int *prefix, int lane) {
+    const bool in_image = px < job.f.width && py < job.f.height;
+    float2 acc_rg = make_float2(0.0f, 0.0f), acc_ba = make_float2(0.0f, 0.0f);
+    unsigned n_inbox = 0, n_shaded = 0;
+    if (in_image)
+        march_ray<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, lut, prefix, acc_rg, acc_ba,
+                                                                   n_inbox, n_shaded);
+    store_pixel(job, px, py, in_image, acc_rg, acc_ba, n_inbox, n_shaded, lane);
 }
 
 // Persistent batch kernel of one variant: normals or not, LUT staged in
@@ -432,6 +448,146 @@ march_single_kernel(const __grid_constant__ SingleParams p) {
     const int py = (t / job.tiles_x) * p.tile_h + (warp / warps_x) * 4 + lane_y(lane);
     march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut + 1 : job.lut,
                                                                 SMEM_LUT ? s_prefix : job.prefix, lane);
+}
+
+// The march of one small render with SPLIT lanes per ray: lane q of a ray
+// evaluates the samples q, q + SPLIT, ..., and all its lanes composite them
+// in order, so every rounding is the one-lane march's.  What a sample adds
+// (Source) does not depend on the samples before it; samples evaluated
+// beyond the ray's end are dropped.
+//
+// A frame of few pixels does not fill the chip: 256^2 are 2048 warps of rays,
+// 3.4 per scheduler, each a serial chain of gathers and shading per sample
+// (issue 37 %).  Here it is SPLIT times the warps with 1/SPLIT of the chain.
+// Each group of samples costs 4 * SPLIT shuffles and as many compositing
+// steps, so a frame that fills the chip is faster with one lane per ray
+// (split_lanes in batch.cu).  A warp is 4x2 (SPLIT 4) or 4x4 pixels.
+template <int LOG2B, int SPLIT, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
+__global__ void __launch_bounds__(kBatchThreads, COMPACT ? 5 : 4)
+march_split_kernel(const __grid_constant__ SingleParams p) {
+    constexpr int B = 1 << LOG2B, ROW = brick_apron(LOG2B), SLICE = ROW * ROW;
+    constexpr int RECS = brick_records(LOG2B);
+    constexpr unsigned kAll = 0xffffffffu, kGroup = (1u << SPLIT) - 1;
+    using Rec = typename RecordOf<COMPACT>::T;
+    extern __shared__ float4 s_dyn[];
+    float4 *s_lut = s_dyn;
+    int *s_prefix = reinterpret_cast<int *>(s_dyn + p.lut_smem_entries + 2);
+    const JobDesc &job = p.job;
+    const MarchFrame &f = job.f;
+    if (SMEM_LUT) {
+        stage_lut(s_lut, s_prefix, job);
+        __syncthreads();
+    }
+    const float4 *lut = SMEM_LUT ? s_lut + 1 : job.lut;
+    const int *prefix = SMEM_LUT ? s_prefix : job.prefix;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & (SPLIT - 1), ray = lane / SPLIT;
+    // the warp's block of pixels in Z-order: 4x2 or 4x4
+    const int t = blockIdx.x;
+    const int px = (t % job.tiles_x) * split_tile_w(SPLIT) + (warp & 1) * 4 + ((ray & 1) | ((ray >> 1) & 2));
+    const int py = (t / job.tiles_x) * split_tile_h(SPLIT) + (warp >> 1) * (8 / SPLIT) +
+                   (((ray >> 1) & 1) | ((ray >> 2) & 2));
+    const bool in_image = px < f.width && py < f.height;
+    float pos[3] = {}, d[3] = {};
+    bool done = !in_image || !setup_ray(f, px, py, pos, d);
+    for (int k = 0; k < q; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) pos[a] = __fadd_rn(pos[a], d[a]);
+    __syncwarp();
+    float2 acc_rg = make_float2(0.0f, 0.0f), acc_ba = make_float2(0.0f, 0.0f);
+    unsigned n_inbox = 0, n_shaded = 0;
+    bool entered = false, clear = false;
+    int cur_brick = -1;
+    const Rec *bp = nullptr;
+    for (int i = 0; __any_sync(kAll, !done); i += SPLIT) {
+        float tc[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) tc[a] = __fmul_rn(__fadd_rn(pos[a], -f.bmin[a]), f.inv_ext[a]);
+        const bool valid = tc[0] >= 0.0f && tc[0] <= 1.0f && tc[1] >= 0.0f && tc[1] <= 1.0f && tc[2] >= 0.0f &&
+                           tc[2] <= 1.0f;
+        // the ray ends here if it has been in the box before, or cannot reach it
+        bool ends = i + q >= f.max_steps;
+        bool never = false;
+        if (!valid)
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                never = never || (tc[a] < 0.0f && d[a] <= 0.0f) || (tc[a] > 1.0f && d[a] >= 0.0f);
+        ends = ends || never;
+        Source s = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+        bool shaded = false;
+        if (valid && !done && !ends) {
+            int k[3];
+            float fr[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float u = __fadd_rn(__fmul_rn(tc[a], f.fext[a]), -0.5f), fl = floorf(u);
+                k[a] = (int)fl + 1;
+                fr[a] = __fadd_rn(u, -fl);
+            }
+            const int id = ((k[0] >> LOG2B) * f.nb[1] + (k[1] >> LOG2B)) * f.nb[2] + (k[2] >> LOG2B);
+            if (id != cur_brick) {
+                cur_brick = id;
+                const uint4 bi = __ldg(job.bricks + id);
+                bp = static_cast<const Rec *>(job.records) + (size_t)bi.x * RECS;
+                clear = job.skip && brick_clear<SMEM_LUT, FAST>(f, make_float2(__uint_as_float(bi.y),
+                                                                               __uint_as_float(bi.z)), prefix);
+            }
+            if (!clear) {
+                const int j = (k[0] & (B - 1)) * SLICE + (k[1] & (B - 1)) * ROW + (k[2] & (B - 1));
+                s = shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST>(f, bp + j, fr[0], fr[1], fr[2], lut);
+                shaded = true;
+            }
+        }
+        // per ray, one bit per sample of the group (the same on all its lanes):
+        // in the box, shaded, and the first one at which the ray ends
+        const unsigned base = lane & ~(SPLIT - 1);
+        const unsigned in = (__ballot_sync(kAll, valid) >> base) & kGroup;
+        const unsigned lit = (__ballot_sync(kAll, shaded) >> base) & kGroup;
+        unsigned stop = (__ballot_sync(kAll, ends) >> base) & kGroup;
+        const unsigned after = entered ? kGroup : ~((in & (0u - in)) * 2 - 1) & (in ? kGroup : 0u);
+        stop |= ~in & after & kGroup;  // outside after having been inside
+        const unsigned before = stop ? (stop & (0u - stop)) - 1 : kGroup;  // the samples in front of it
+        entered = entered || in != 0;
+        unsigned taken = 0;
+#pragma unroll
+        for (int k = 0; k < SPLIT; ++k) {
+            const Source sk = {make_float2(__shfl_sync(kAll, s.rg.x, k, SPLIT), __shfl_sync(kAll, s.rg.y, k, SPLIT)),
+                               make_float2(__shfl_sync(kAll, s.ba.x, k, SPLIT), __shfl_sync(kAll, s.ba.y, k, SPLIT))};
+            if (!done && acc_ba.y < 0.99f && ((before >> k) & 1)) {
+                taken |= 1u << k;
+                if ((lit >> k) & 1) composite<FAST>(sk, acc_rg, acc_ba);
+            }
+        }
+        n_inbox += __popc(taken & in);
+        n_shaded += __popc(taken & lit);
+        done = done || stop != 0 || !(acc_ba.y < 0.99f);
+#pragma unroll
+        for (int k = 0; k < SPLIT; ++k)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) pos[a] = __fadd_rn(pos[a], d[a]);
+    }
+    const bool writes = in_image && q == 0;
+    store_pixel(job, px, py, writes, acc_rg, acc_ba, writes ? n_inbox : 0, writes ? n_shaded : 0, lane);
+}
+
+template <int LOG2B, int SPLIT, bool FAST>
+const void *split_variant_of(int v) {
+    switch (v & 7) {
+    case 0: return (const void *)march_split_kernel<LOG2B, SPLIT, false, false, false, FAST>;
+    case 1: return (const void *)march_split_kernel<LOG2B, SPLIT, true, false, false, FAST>;
+    case 2: return (const void *)march_split_kernel<LOG2B, SPLIT, false, true, false, FAST>;
+    case 3: return (const void *)march_split_kernel<LOG2B, SPLIT, true, true, false, FAST>;
+    case 4: return (const void *)march_split_kernel<LOG2B, SPLIT, false, false, true, FAST>;
+    case 5: return (const void *)march_split_kernel<LOG2B, SPLIT, true, false, true, FAST>;
+    case 6: return (const void *)march_split_kernel<LOG2B, SPLIT, false, true, true, FAST>;
+    default: return (const void *)march_split_kernel<LOG2B, SPLIT, true, true, true, FAST>;
+    }
+}
+
+template <int LOG2B>
+const void *split_kernel_log2(int lanes, int v) {
+    if (lanes == 4)
+        return (v & kSingleFast) ? split_variant_of<LOG2B, 4, true>(v) : split_variant_of<LOG2B, 4, false>(v);
+    return (v & kSingleFast) ? split_variant_of<LOG2B, 2, true>(v) : split_variant_of<LOG2B, 2, false>(v);
 }
 
 template <int LOG2B, int UNROLL, bool FAST>

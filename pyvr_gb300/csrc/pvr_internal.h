@@ -115,6 +115,14 @@ constexpr int kSingleNormals = 1, kSingleSmemLut = 2, kSingleCompact = 4, kSingl
 constexpr int kMaxSmemLut = 2048;
 const void *batch_kernel(int log2b, const Tuning &t, int variant);
 const void *single_kernel(int log2b, const Tuning &t, int variant);
+// The kernel for one small render with 2 or 4 lanes per ray, and the pixels of
+// one of its blocks.
+const void *split_kernel(int log2b, int lanes, int variant);
+// Whether launches of this batch may use it: not beside others on the device,
+// where several lanes per ray cost throughput.
+void batch_allow_split(pvr_batch *b, bool allow);
+__host__ __device__ constexpr int split_tile_w(int) { return 8; }
+__host__ __device__ constexpr int split_tile_h(int lanes) { return 32 / lanes; }
 size_t batch_smem_bytes(int lut_smem_entries);
 int max_batch_blocks_per_sm(int log2b, const Tuning &t, int lut_smem_entries, int variant);
 // the variant bits of a job before it is filled

@@ -271,6 +271,8 @@ void scheduler_loop(pvr_server *srv) {
             s.reqs.push_back(q);
             srv->queue.pop_front();
         }
+        // a render with the device to itself may take several lanes per ray
+        pvr::batch_allow_split(s.batch, srv->n_inflight == 1 && srv->queue.empty());
         lk.unlock();
         const long long t_launch = now_ns();
         for (auto &q : s.reqs) q.t_launch = t_launch;

@@ -1,0 +1,79 @@
+"""Small single renders with 2 or 4 lanes per ray: images, float images and
+sample counts equal the oracle's (exact arithmetic, bit for bit) and those of
+the persistent batch kernel, which marches one lane per ray (both
+arithmetics)."""
+
+import numpy as np
+import pytest
+
+import oracle
+from pyvr_gb300 import Camera, Light, RenderConfig, Volume
+from pyvr_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+# 4 lanes up to 224^2 pixels on 152 SMs, 2 up to 384^2
+SIZES = [(1, 1), (9, 5), (61, 37), (224, 224), (225, 225), (301, 233)]
+
+
+def _render(dv, lut, cam, cfg, w, h, alone):
+    from pyvr_gb300.batch import BatchRenderer, RenderJob
+    o8 = [torch.zeros(w * h * 4, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    of = [torch.zeros(w * h * 4, dtype=torch.float32, device="cuda") for _ in range(2)]
+    n = torch.zeros((2, 2), dtype=torch.int64, device="cuda")
+    jobs = [RenderJob(dv, lut, cam, Light.directional([1, -1, 0], 0.2, 0.8), cfg, w, h, o8[k], of[k], n[k])
+            for k in range(1 if alone else 2)]
+    br = BatchRenderer(capacity=2, slots=1)
+    torch.cuda.synchronize()
+    br.render(jobs)
+    br.synchronize()
+    br.close()
+    return o8[0].cpu().numpy(), of[0].cpu().numpy(), n[0].tolist()
+
+
+@pytest.mark.parametrize("normals", ["device", "none"])
+@pytest.mark.parametrize("records,dtype", [("float", "f32"), ("half_normals", "u8")])
+@pytest.mark.parametrize("lut_size", [256, 4096])
+def test_split_march(normals, records, dtype, lut_size):
+    from pyvr_gb300.batch import DeviceLUT, DeviceVolume, arithmetic, get_compact_records, set_compact_records
+    from pyvr_gb300.renderer import rgba_lut
+    noise = W.value_noise((24, 24, 24), 4)
+    noise[noise < 0.4] = 0.0  # clear bricks and flat places
+    data = W.to_storage(noise, dtype)
+    vol = Volume(data=data, min_bounds=np.full(3, -1.0, np.float32), max_bounds=np.full(3, 1.0, np.float32))
+    vs = 1.0 / 255.0 if dtype == "u8" else 1.0
+    prev = get_compact_records()
+    set_compact_records(records)
+    try:
+        dv = DeviceVolume(vol, value_scale=vs, normals=normals, brick_log2=2)
+    finally:
+        set_compact_records(prev)
+    if normals == "device":
+        vol.normals = dv.read_normals()
+    from pyvr_gb300 import OpacityTransferFunction
+    otf = OpacityTransferFunction([(0.0, 0.0), (0.1, 0.0), (0.5, 0.3), (1.0, 0.9)])
+    ctf = W.standin_colormap(5)
+    lut, table = DeviceLUT(ctf, otf, lut_size), rgba_lut(ctf, otf, lut_size)
+    outside = Camera.from_spherical(np.zeros(3, np.float32), 0.7, 0.3, 0.0, 3.0)
+    inside = Camera.from_spherical(np.zeros(3, np.float32), 2.0, -0.2, 0.0, 0.4)
+    configs = [(RenderConfig.balanced(), s) for s in SIZES]
+    # step limits inside a group of samples, and steps so long that a ray has few samples
+    configs += [(RenderConfig.custom(0.02, m), (31, 17)) for m in (1, 2, 3, 4, 5, 7)]
+    configs += [(RenderConfig.custom(0.7, 9), (31, 17))]
+    for cfg, (w, h) in configs:
+        for cam in (outside, inside):
+            for mode in ("exact", "fast"):
+                with arithmetic(mode):
+                    a8, af, an = _render(dv, lut, cam, cfg, w, h, True)
+                    b8, bf, bn = _render(dv, lut, cam, cfg, w, h, False)
+                assert np.array_equal(a8, b8) and np.array_equal(af.view(np.uint32), bf.view(np.uint32)), (w, h, mode)
+                assert an == bn, (w, h, mode)
+                if mode == "exact" and w <= 61:
+                    s = W.frame_inputs(vol, cam, Light.directional([1, -1, 0], 0.2, 0.8), cfg, table, w, h, vs,
+                                       batch_camera=True)
+                    o8, of, on = oracle.render(s)
+                    assert np.array_equal(a8.reshape(o8.shape), o8) and an[0] == on
+                    assert np.array_equal(af.reshape(of.shape).view(np.uint32), of.view(np.uint32))
+    dv.close()
