@@ -10,6 +10,7 @@ tensors (plumbing only: the kernels are the library's).
 from __future__ import annotations
 
 import ctypes
+from array import array
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -275,13 +276,15 @@ class DeviceLUT:
         queued on ``stream``): the same float32 entries as ``rgba_lut`` computes
         on the host.  No batch reading this LUT may be in flight."""
         n = int(size or max(color_tf.lut_size, opacity_tf.lut_size))
-        cx = np.ascontiguousarray([float(p[0]) for p in color_tf.control_points], np.float64)
-        crgb = np.ascontiguousarray([[float(c) for c in p[1]] for p in color_tf.control_points], np.float64)
-        ox = np.ascontiguousarray([float(p[0]) for p in opacity_tf.control_points], np.float64)
-        oa = np.ascontiguousarray([float(p[1]) for p in opacity_tf.control_points], np.float64)
+        cx = array("d", [p[0] for p in color_tf.control_points])
+        crgb = array("d", [c for p in color_tf.control_points for c in p[1]])
+        ox = array("d", [p[0] for p in opacity_tf.control_points])
+        oa = array("d", [p[1] for p in opacity_tf.control_points])
+        if len(crgb) != 3 * len(cx):
+            raise ValueError("colours must have three components")
         s = getattr(stream, "cuda_stream", stream)
-        check(_lib().pvr_lut_build(self.handle, cx.ctypes.data, crgb.ctypes.data, len(cx), ox.ctypes.data,
-                                   oa.ctypes.data, len(ox), n, s))
+        check(_lib().pvr_lut_build(self.handle, *(a.buffer_info()[0] for a in (cx, crgb)), len(cx),
+                                   *(a.buffer_info()[0] for a in (ox, oa)), len(ox), n, s))
         self.size = n
 
     def read(self) -> np.ndarray:
