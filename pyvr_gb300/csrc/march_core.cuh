@@ -67,12 +67,47 @@ __device__ __forceinline__ float2 half_pair(uint32_t b) {
     return __half22float2(h);
 }
 
-// {value, nx, ny, nz} of one record
-__device__ __forceinline__ float4 load_rec(const float4 *p) { return __ldg(p); }
-__device__ __forceinline__ float4 load_rec(const uint2 *p) {
-    const uint2 r = __ldg(p);
-    const float2 a = half_pair(r.x), b = half_pair(r.y);
-    return make_float4(a.x, a.y, b.x, b.y);
+// How the lerps of a sample's records are written: the same two roundings per
+// lerp and lane in each.  Packed: two lanes per instruction.  Scalar: fewer
+// register pairs, for the kernel that has 40 registers.  Mixed: the first
+// lerp's difference b - a takes b as a half (one instruction of a half and a
+// float), so that only a is converted.  Measured per kernel, us (seeds of
+// the single and batch cases): half records at 40 registers packed 80.5 /
+// 135.6 / 143, scalar 76.3 / 131.5 / 136, mixed 94 / 141 / 160 (spills);
+// batches at 48 and 64 registers packed 1498 / 1526 / 1689, mixed 1441 / 1459
+// / 1638.
+enum LerpForm { kLerpPacked = 0, kLerpScalar = 1, kLerpMixed = 2 };
+
+template <int LERP>
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float t) {
+    if (LERP == kLerpScalar) return make_float2(lerp_tex(a.x, b.x, t), lerp_tex(a.y, b.y, t));
+    return lerp_tex2(a, b, t);
+}
+template <int LERP>
+__device__ __forceinline__ float4 lerp4(float4 a, float4 b, float t) {
+    const float2 x = lerp2<LERP>(lo2(a), lo2(b), t), y = lerp2<LERP>(hi2(a), hi2(b), t);
+    return make_float4(x.x, x.y, y.x, y.y);
+}
+// half h (the low 16 bits) - c, rounded once
+__device__ __forceinline__ float sub_half(uint32_t h, float c) {
+    float d;
+    asm("sub.rn.f32.f16 %0, %1, %2;" : "=f"(d) : "h"((unsigned short)h), "f"(c));
+    return d;
+}
+// {value, nx, ny, nz} between two records
+template <int LERP>
+__device__ __forceinline__ float4 lerp_rec(float4 a, float4 b, float t) { return lerp4<LERP>(a, b, t); }
+template <int LERP>
+__device__ __forceinline__ float4 lerp_rec(uint2 a, uint2 b, float t) {
+    const float2 a0 = half_pair(a.x), a1 = half_pair(a.y);
+    if (LERP == kLerpMixed) {
+        const float2 d0 = make_float2(sub_half(b.x, a0.x), sub_half(b.x >> 16, a0.y));
+        const float2 d1 = make_float2(sub_half(b.y, a1.x), sub_half(b.y >> 16, a1.y));
+        const float2 x = __ffma2_rn(dup2(t), d0, a0), y = __ffma2_rn(dup2(t), d1, a1);
+        return make_float4(x.x, x.y, y.x, y.y);
+    }
+    const float2 b0 = half_pair(b.x), b1 = half_pair(b.y);
+    return lerp4<LERP>(make_float4(a0.x, a0.y, a1.x, a1.y), make_float4(b0.x, b0.y, b1.x, b1.y), t);
 }
 // the stored value of one record
 __device__ __forceinline__ float load_value(const float4 *p) { return __ldg(reinterpret_cast<const float *>(p)); }
@@ -116,35 +151,30 @@ __device__ __forceinline__ void composite(const Source &s, float2 &acc_rg, float
 
 // Shading of one in-box sample (frag:93-110).  p: the record of the
 // footprint's lower corner; fx, fy, fz: the filter fractions.
-template <int LOG2B, bool NORMALS, bool SMEM_LUT, bool FAST, typename Rec>
+template <int LOG2B, bool NORMALS, bool SMEM_LUT, bool FAST, int LERP, typename Rec>
 __device__ __forceinline__ Source shade_sample(const MarchFrame &f, const Rec *__restrict__ p,
                                                float fx, float fy, float fz, const float4 *lut) {
     constexpr int ROW = brick_apron(LOG2B), SLICE = ROW * ROW;
     float density;
     float n[3];
     if (NORMALS) {
-        const float4 r000 = load_rec(p);
-        const float4 r001 = load_rec(p + 1);
-        const float4 r010 = load_rec(p + ROW);
-        const float4 r011 = load_rec(p + ROW + 1);
-        const float4 r100 = load_rec(p + SLICE);
-        const float4 r101 = load_rec(p + SLICE + 1);
-        const float4 r110 = load_rec(p + SLICE + ROW);
-        const float4 r111 = load_rec(p + SLICE + ROW + 1);
+        const Rec r000 = __ldg(p);
+        const Rec r001 = __ldg(p + 1);
+        const Rec r010 = __ldg(p + ROW);
+        const Rec r011 = __ldg(p + ROW + 1);
+        const Rec r100 = __ldg(p + SLICE);
+        const Rec r101 = __ldg(p + SLICE + 1);
+        const Rec r110 = __ldg(p + SLICE + ROW);
+        const Rec r111 = __ldg(p + SLICE + ROW + 1);
         // texture(volume_texture, tex.zyx) and texture(normal_volume, ...):
         // lerp along z, then y, then x; lanes (value, nx) and (ny, nz)
-        const float2 a = lerp_tex2(lerp_tex2(lerp_tex2(lo2(r000), lo2(r001), fz),
-                                             lerp_tex2(lo2(r010), lo2(r011), fz), fy),
-                                   lerp_tex2(lerp_tex2(lo2(r100), lo2(r101), fz),
-                                             lerp_tex2(lo2(r110), lo2(r111), fz), fy), fx);
-        const float2 b = lerp_tex2(lerp_tex2(lerp_tex2(hi2(r000), hi2(r001), fz),
-                                             lerp_tex2(hi2(r010), hi2(r011), fz), fy),
-                                   lerp_tex2(lerp_tex2(hi2(r100), hi2(r101), fz),
-                                             lerp_tex2(hi2(r110), hi2(r111), fz), fy), fx);
-        density = __fmul_rn(a.x, f.value_scale);
-        n[0] = a.y;
-        n[1] = b.x;
-        n[2] = b.y;
+        const float4 v = lerp4<LERP>(lerp4<LERP>(lerp_rec<LERP>(r000, r001, fz), lerp_rec<LERP>(r010, r011, fz), fy),
+                                     lerp4<LERP>(lerp_rec<LERP>(r100, r101, fz), lerp_rec<LERP>(r110, r111, fz), fy),
+                                     fx);
+        density = __fmul_rn(v.x, f.value_scale);
+        n[0] = v.y;
+        n[1] = v.z;
+        n[2] = v.w;
     } else {
         const float v000 = load_value(p), v001 = load_value(p + 1);
         const float v010 = load_value(p + ROW), v011 = load_value(p + ROW + 1);
@@ -179,8 +209,8 @@ __device__ __forceinline__ Source shade_sample(const MarchFrame &f, const Rec *_
         A = __ldg(lut + lut_index(lfl, f.flut_max));
         B = __ldg(lut + lut_index(__fadd_rn(lfl, 1.0f), f.flut_max));
     }
-    const float2 crg = lerp_tex2(lo2(A), lo2(B), la);
-    const float2 cba = lerp_tex2(hi2(A), hi2(B), la);  // (blue, alpha_tf)
+    const float2 crg = lerp2<LERP>(lo2(A), lo2(B), la);
+    const float2 cba = lerp2<LERP>(hi2(A), hi2(B), la);  // (blue, alpha_tf)
 
     if (FAST) {
         // alpha = 1 - exp(-alpha_tf * step/ref) (frag:101)
@@ -241,8 +271,10 @@ __device__ __forceinline__ bool brick_clear(const MarchFrame &f, float2 m, const
     return prefix_entry<SMEM_LUT>(prefix, ihi + 1) == prefix_entry<SMEM_LUT>(prefix, ilo);
 }
 
-// One pixel's ray of volume.frag.glsl:main (lines 70-122).
-template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
+// One pixel's ray of volume.frag.glsl:main (lines 70-122).  PACKED: the x and
+// y coordinates in packed instructions (their frame constants then take six
+// registers); scalar ones read the constants from the parameter bank.
+template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST, int LERP, bool PACKED>
 __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, const float4 *lut,
                                           const int *prefix, float2 &acc_rg, float2 &acc_ba,
                                           unsigned &n_inbox, unsigned &n_shaded) {
@@ -272,7 +304,9 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
         for (int u = 0; u < UNROLL; ++u) {
             if (!(i < f.max_steps && acc_ba.y < 0.99f)) return;
             // world_to_texture_coords (frag:25-27, 88)
-            const float2 txy = __fmul2_rn(__fadd2_rn(pxy, nbmin_xy), inv_xy);
+            const float2 txy = PACKED ? __fmul2_rn(__fadd2_rn(pxy, nbmin_xy), inv_xy)
+                                      : make_float2(__fmul_rn(__fadd_rn(pxy.x, -f.bmin[0]), f.inv_ext[0]),
+                                                    __fmul_rn(__fadd_rn(pxy.y, -f.bmin[1]), f.inv_ext[1]));
             const float tz = __fmul_rn(__fadd_rn(pz, nbmin_z), inv_z);
             const bool valid = txy.x >= 0.0f && txy.x <= 1.0f && txy.y >= 0.0f &&
                                txy.y <= 1.0f && tz >= 0.0f && tz <= 1.0f;
@@ -280,7 +314,8 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
                 entered = true;
                 ++n_inbox;
                 // texel coordinate u = t*size - 0.5, lower texel k = floor(u)
-                const float2 sxy = __fmul2_rn(txy, fext_xy);
+                const float2 sxy = PACKED ? __fmul2_rn(txy, fext_xy)
+                                          : make_float2(__fmul_rn(txy.x, f.fext[0]), __fmul_rn(txy.y, f.fext[1]));
                 const float ux = __fadd_rn(sxy.x, -0.5f), uy = __fadd_rn(sxy.y, -0.5f);
                 const float uz = __fadd_rn(__fmul_rn(tz, fext_z), -0.5f);
                 const float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
@@ -298,7 +333,7 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
                 if (!clear) {
                     ++n_shaded;
                     const int j = (kx & (B - 1)) * SLICE + (ky & (B - 1)) * ROW + (kz & (B - 1));
-                    composite<FAST>(shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST>(
+                    composite<FAST>(shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST, LERP>(
                                         f, bp + j, __fadd_rn(ux, -flx), __fadd_rn(uy, -fly), __fadd_rn(uz, -flz), lut),
                                     acc_rg, acc_ba);
                 }
@@ -333,8 +368,8 @@ __device__ __forceinline__ int lane_y(int lane) { return ((lane >> 1) & 1) | ((l
 // counts in shared memory.
 __device__ __forceinline__ void stage_lut(float4 *s_lut, int *s_prefix, const JobDesc &job) {
     const int size = job.f.lut_size;
-    for (int k = threadIdx.x; k < size + 2; k += kBatchThreads) s_lut[k] = job.lut[min(max(k - 1, 0), size - 1)];
-    for (int k = threadIdx.x; k <= size; k += kBatchThreads) s_prefix[k] = job.prefix[k];
+    for (int k = threadIdx.x; k < size + 2; k += blockDim.x) s_lut[k] = job.lut[min(max(k - 1, 0), size - 1)];
+    for (int k = threadIdx.x; k <= size; k += blockDim.x) s_prefix[k] = job.prefix[k];
 }
 
 // Writes the lane's pixel (writes: it has one) and adds the warp's sample
@@ -360,15 +395,15 @@ __device__ __forceinline__ void store_pixel(const JobDesc &job, int px, int py, 
     }
 }
 
-template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
+template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST, int LERP, bool PACKED>
 __device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, const float4 *lut,
                                            const int *prefix, int lane) {
     const bool in_image = px < job.f.width && py < job.f.height;
     float2 acc_rg = make_float2(0.0f, 0.0f), acc_ba = make_float2(0.0f, 0.0f);
     unsigned n_inbox = 0, n_shaded = 0;
     if (in_image)
-        march_ray<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, lut, prefix, acc_rg, acc_ba,
-                                                                   n_inbox, n_shaded);
+        march_ray<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, LERP, PACKED>(job, px, py, lut, prefix, acc_rg,
+                                                                                 acc_ba, n_inbox, n_shaded);
     store_pixel(job, px, py, in_image, acc_rg, acc_ba, n_inbox, n_shaded, lane);
 }
 
@@ -417,8 +452,8 @@ march_batch_kernel(const __grid_constant__ BatchParams p) {
         const int local = t - job.tile_base;
         const int px = (local % job.tiles_x) * p.tile_w + sub_x;
         const int py = (local / job.tiles_x) * p.tile_h + sub_y;
-        march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut + 1 : job.lut,
-                                                                    SMEM_LUT ? s_prefix : job.prefix, lane);
+        march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, COMPACT ? kLerpMixed : kLerpPacked, false>(
+            job, px, py, SMEM_LUT ? s_lut + 1 : job.lut, SMEM_LUT ? s_prefix : job.prefix, lane);
         __syncthreads();  // s_tile / the staged LUT are rewritten next round
     }
 }
@@ -446,8 +481,8 @@ march_single_kernel(const __grid_constant__ SingleParams p) {
     const int t = blockIdx.x;
     const int px = (t % job.tiles_x) * p.tile_w + (warp % warps_x) * 8 + lane_x(lane);
     const int py = (t / job.tiles_x) * p.tile_h + (warp / warps_x) * 4 + lane_y(lane);
-    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST>(job, px, py, SMEM_LUT ? s_lut + 1 : job.lut,
-                                                                SMEM_LUT ? s_prefix : job.prefix, lane);
+    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, COMPACT ? kLerpScalar : kLerpPacked, true>(
+        job, px, py, SMEM_LUT ? s_lut + 1 : job.lut, SMEM_LUT ? s_prefix : job.prefix, lane);
 }
 
 // The march of one small render with SPLIT lanes per ray: lane q of a ray
@@ -533,7 +568,7 @@ march_split_kernel(const __grid_constant__ SingleParams p) {
             }
             if (!clear) {
                 const int j = (k[0] & (B - 1)) * SLICE + (k[1] & (B - 1)) * ROW + (k[2] & (B - 1));
-                s = shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST>(f, bp + j, fr[0], fr[1], fr[2], lut);
+                s = shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST, kLerpPacked>(f, bp + j, fr[0], fr[1], fr[2], lut);
                 shaded = true;
             }
         }

@@ -43,10 +43,9 @@ __device__ __forceinline__ float lerp_tex(float a, float b, float t) {
 }
 
 // Two lerps at once with the packed FP32x2 pipe (sm_100+): per lane the
-// same two IEEE round-to-nearest operations as lerp_tex (b - a is formed
-// exactly as fma(a, -1, b)).
+// same two IEEE round-to-nearest operations as lerp_tex.
 __device__ __forceinline__ float2 lerp_tex2(float2 a, float2 b, float t) {
-    return __ffma2_rn(make_float2(t, t), __ffma2_rn(a, make_float2(-1.0f, -1.0f), b), a);
+    return __ffma2_rn(make_float2(t, t), __fadd2_rn(b, make_float2(-a.x, -a.y)), a);
 }
 
 // exp(x): k = rint(x/ln2), r = x - k*ln2 with ln2 split 0.693359375 +
