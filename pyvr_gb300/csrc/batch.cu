@@ -170,17 +170,25 @@ int build_graph(Slot &s, const LaunchKey &key, void **args) {
     return PVR_OK;
 }
 
-// Lanes per ray of a single render that has the chip to itself, by its pixels
-// per SM.  Device us with 1 / 2 / 4 lanes, 256^3 uint8 in float records and
-// 384^3 float16 in half records (balanced), 64^3 float32 (high quality):
+// Lanes per ray of a single render that has the chip to itself: 4 or 2 where
+// all blocks of that kernel are resident at once (its launch bounds: 5 per SM
+// for half records, 4 for float ones), else 1.  Device us with 1 / 2 / 4 lanes,
+// 256^3 uint8 in float records, 384^3 float16 in half records (balanced) and
+// 64^3 float32 (high quality):
 //   192^2   59.8 / 40.2 / 38.7    79.5 / 41.1 / 34.9    63.6 / 44.2 / 36.8
 //   256^2   64.3 / 55.1 / 59.1    84.0 / 53.7 / 52.4    65.0 / 57.7 / 53.5
 //   384^2   78.5 / 78.2 / 87.5    93.9 / 83.1 / 81.2    87.4 / 85.5 / 89.5
 //   512^2  102.7 / 103.7 / 130   103.5 / 104.5 / 117   122.7 / 125.7 / 142
-constexpr int kSplit4Pixels = 330, kSplit2Pixels = 970;  // 224^2 and 384^2 on 152 SMs
-int split_lanes(int width, int height, int sms) {
-    const long long pixels = (long long)width * height;
-    return pixels <= (long long)kSplit4Pixels * sms ? 4 : pixels <= (long long)kSplit2Pixels * sms ? 2 : 1;
+// A second wave of blocks loses where most rays hit the box (153x938: 46.0 us
+// with 1 lane, 54.2 with 2); in one wave 102 random frames of up to 10^5 pixels
+// were 1.5 times as fast on average, the worst 0.93 (16.6 -> 17.7 us).
+int split_lanes(int width, int height, int sms, bool compact) {
+    for (int lanes = 4; lanes >= 2; lanes /= 2) {
+        const int tw = pvr::split_tile_w(lanes), th = pvr::split_tile_h(lanes);
+        const long long tiles = (long long)((width + tw - 1) / tw) * ((height + th - 1) / th);
+        if (tiles <= (long long)sms * pvr::split_blocks_per_sm(compact)) return lanes;
+    }
+    return 1;
 }
 
 // One launch over jobs[idx[0..n)] (jobs of one variant, at most
@@ -201,7 +209,7 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
         // launched directly (its parameters are copied at the launch, and it
         // uses no work counter); the slot's event tracks it like a batch
         pvr::SingleParams &sp = b->single;
-        const int lanes = b->split ? split_lanes(jobs[0].width, jobs[0].height, b->sms) : 1;
+        const int lanes = b->split ? split_lanes(jobs[0].width, jobs[0].height, b->sms, jobs[0].volume->compact) : 1;
         const int tile_w = lanes > 1 ? pvr::split_tile_w(lanes) : b->tuning.tile_w;
         const int tile_h = lanes > 1 ? pvr::split_tile_h(lanes) : b->tuning.tile_h;
         if (int rc = pvr::fill_job(jobs[0], tile_w, tile_h, fast, sp.job)) return rc;

@@ -498,7 +498,7 @@ march_single_kernel(const __grid_constant__ SingleParams p) {
 // steps, so a frame that fills the chip is faster with one lane per ray
 // (split_lanes in batch.cu).  A warp is 4x2 (SPLIT 4) or 4x4 pixels.
 template <int LOG2B, int SPLIT, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
-__global__ void __launch_bounds__(kBatchThreads, COMPACT ? 5 : 4)
+__global__ void __launch_bounds__(kBatchThreads, split_blocks_per_sm(COMPACT))
 march_split_kernel(const __grid_constant__ SingleParams p) {
     constexpr int B = 1 << LOG2B, ROW = brick_apron(LOG2B), SLICE = ROW * ROW;
     constexpr int RECS = brick_records(LOG2B);

@@ -121,6 +121,7 @@ const void *split_kernel(int log2b, int lanes, int variant);
 // Whether launches of this batch may use it: not beside others on the device,
 // where several lanes per ray cost throughput.
 void batch_allow_split(pvr_batch *b, bool allow);
+__host__ __device__ constexpr int split_blocks_per_sm(bool compact) { return compact ? 5 : 4; }
 __host__ __device__ constexpr int split_tile_w(int) { return 8; }
 __host__ __device__ constexpr int split_tile_h(int lanes) { return 32 / lanes; }
 size_t batch_smem_bytes(int lut_smem_entries);

@@ -14,8 +14,9 @@ pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
 
-# 4 lanes up to 224^2 pixels on 152 SMs, 2 up to 384^2
-SIZES = [(1, 1), (9, 5), (61, 37), (224, 224), (225, 225), (301, 233)]
+# 4 lanes up to about 197^2 (220^2 with half records) pixels on 152 SMs, 2 up to
+# 279^2 (312^2)
+SIZES = [(1, 1), (9, 5), (61, 37), (192, 200), (224, 224), (301, 233)]
 
 
 def _render(dv, lut, cam, cfg, w, h, alone):
