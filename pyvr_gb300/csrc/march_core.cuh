@@ -57,6 +57,7 @@ __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); 
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
+// {value, nx, ny, nz}; without normals a quad of values (layout.cu)
 template <bool COMPACT> struct RecordOf { using T = float4; };
 template <> struct RecordOf<true> { using T = uint2; };
 
@@ -109,10 +110,16 @@ __device__ __forceinline__ float4 lerp_rec(uint2 a, uint2 b, float t) {
     const float2 b0 = half_pair(b.x), b1 = half_pair(b.y);
     return lerp4<LERP>(make_float4(a0.x, a0.y, a1.x, a1.y), make_float4(b0.x, b0.y, b1.x, b1.y), t);
 }
-// the stored value of one record
-__device__ __forceinline__ float load_value(const float4 *p) { return __ldg(reinterpret_cast<const float *>(p)); }
-__device__ __forceinline__ float load_value(const uint2 *p) {
-    return __half2float(__ldg(reinterpret_cast<const __half *>(p)));
+// A record without normals is the quad of values {(y, z), (y + 1, z),
+// (y, z + 1), (y + 1, z + 1)}: its lerp along z, lanes y and y + 1.
+template <int LERP>
+__device__ __forceinline__ float2 lerp_quad(float4 q, float t) { return lerp2<LERP>(lo2(q), hi2(q), t); }
+template <int LERP>
+__device__ __forceinline__ float2 lerp_quad(uint2 q, float t) {
+    const float2 a = half_pair(q.x);
+    if (LERP == kLerpMixed)
+        return __ffma2_rn(dup2(t), make_float2(sub_half(q.y, a.x), sub_half(q.y >> 16, a.y)), a);
+    return lerp2<LERP>(a, half_pair(q.y), t);
 }
 
 template <bool SMEM>
@@ -176,13 +183,9 @@ __device__ __forceinline__ Source shade_sample(const MarchFrame &f, const Rec *_
         n[1] = v.z;
         n[2] = v.w;
     } else {
-        const float v000 = load_value(p), v001 = load_value(p + 1);
-        const float v010 = load_value(p + ROW), v011 = load_value(p + ROW + 1);
-        const float v100 = load_value(p + SLICE), v101 = load_value(p + SLICE + 1);
-        const float v110 = load_value(p + SLICE + ROW), v111 = load_value(p + SLICE + ROW + 1);
-        const float2 zz0 = lerp_tex2(make_float2(v000, v010), make_float2(v001, v011), fz);
-        const float2 zz1 = lerp_tex2(make_float2(v100, v110), make_float2(v101, v111), fz);
-        const float2 yy = lerp_tex2(make_float2(zz0.x, zz1.x), make_float2(zz0.y, zz1.y), fy);
+        const Rec q0 = __ldg(p), q1 = __ldg(p + SLICE);
+        const float2 zz0 = lerp_quad<LERP>(q0, fz), zz1 = lerp_quad<LERP>(q1, fz);
+        const float2 yy = lerp2<LERP>(make_float2(zz0.x, zz1.x), make_float2(zz0.y, zz1.y), fy);
         density = __fmul_rn(lerp_tex(yy.x, yy.y, fx), f.value_scale);
         // the reference's unbound normal sampler reads the R32F volume
         // texture: normal = (density, 0, 0)

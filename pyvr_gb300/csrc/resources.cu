@@ -608,6 +608,10 @@ int pvr_volume_read_normals(const pvr_volume *v, float *normals_out) {
     if (!v->layout_ready) return fail(PVR_ERR_STATE, "volume layout not built");
     if (v->ready) PVR_CUDA(cudaEventSynchronize(v->ready));
     const size_t n = (size_t)v->dims[0] * v->dims[1] * v->dims[2] * 3;
+    if (v->normals_mode == PVR_NORMALS_NONE) {  // its records hold no normals
+        std::memset(normals_out, 0, n * sizeof(float));
+        return PVR_OK;
+    }
     float *d = nullptr;
     PVR_CUDA(cudaMalloc(&d, n * sizeof(float)));
     cudaError_t e = pvr::launch_read_normals(v->geo, v->dims, v->d_bricks, v->d_records, v->compact, d, 0);
