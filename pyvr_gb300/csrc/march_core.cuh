@@ -236,7 +236,7 @@ __device__ __forceinline__ Source shade_sample(const MarchFrame &f, const Rec *_
     if (n2 > 0.0f) {
         // normalize(n) = n * rsqrt(n.n), the reciprocal square root rounded
         // once (correctly rounded: equal to RN(1/sqrt(x)) evaluated in double)
-        const float inv = __frsqrt_rn(n2);
+        const float inv = rsqrt_rn(n2);
         const float d = __fadd_rn(__fadd_rn(__fmul_rn(__fmul_rn(n[0], inv), f.light_dir[0]),
                                             __fmul_rn(__fmul_rn(n[1], inv), f.light_dir[1])),
                                   __fmul_rn(__fmul_rn(n[2], inv), f.light_dir[2]));
@@ -469,7 +469,7 @@ march_batch_kernel(const __grid_constant__ BatchParams p) {
 // records need 16 fewer registers for a sample's 8 records: those variants
 // run 6 blocks per SM (40 registers) instead of 5 (48).
 template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
-__global__ void __launch_bounds__(kBatchThreads, COMPACT ? 6 : 5)
+__global__ void __launch_bounds__(kBatchThreads, NORMALS ? (COMPACT ? 6 : 5) : 6)
 march_single_kernel(const __grid_constant__ SingleParams p) {
     extern __shared__ float4 s_dyn[];
     float4 *s_lut = s_dyn;

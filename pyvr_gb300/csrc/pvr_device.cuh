@@ -51,14 +51,11 @@ __device__ __forceinline__ float2 lerp_tex2(float2 a, float2 b, float t) {
 // exp(x): k = rint(x/ln2), r = x - k*ln2 with ln2 split 0.693359375 +
 // -2.12194440e-4 (Cody & Waite), exp(r) by its Taylor series to r^7
 // (|r| <= ln2/2, truncation < 0.1 ulp), scaled by 2^k.  Flushes to 0 below
-// -87.3 (where 1 - exp(x) is already 1.0f).
-__device__ __forceinline__ float pvr_expf(float x) {
-    if (x != x) return x;
-    if (x > 88.72283f) return __int_as_float(0x7f800000);
-    if (x < -87.33654f) return 0.0f;
-    float kf = rintf(x * 1.44269504f);
-    float r = fmaf(kf, -0.693359375f, x);
-    r = fmaf(kf, 2.12194440e-4f, r);
+// -87.3 (where 1 - exp(x) is already 1.0f).  For |x| <= 87 (every opacity
+// short of 87) k comes from the low bits of x/ln2 + 1.5 * 2^23, whose rounding
+// is the rint, and 2^k is one shift of them: 32 -> 20 issue cycles per warp;
+// the tests compare it with the rint form for every float.
+__device__ __forceinline__ float exp_taylor(float r) {
     float p = 1.98412698e-4f;
     p = fmaf(p, r, 1.38888889e-3f);
     p = fmaf(p, r, 8.33333333e-3f);
@@ -66,12 +63,27 @@ __device__ __forceinline__ float pvr_expf(float x) {
     p = fmaf(p, r, 1.66666667e-1f);
     p = fmaf(p, r, 0.5f);
     p = fmaf(p, r, 1.0f);
-    p = fmaf(p, r, 1.0f);
+    return fmaf(p, r, 1.0f);
+}
+__device__ __forceinline__ float exp_reduced(float x, float kf) {
+    return exp_taylor(fmaf(kf, 2.12194440e-4f, fmaf(kf, -0.693359375f, x)));
+}
+static __device__ __noinline__ float exp_edges(float x) {
+    if (x != x) return x;
+    if (x > 88.72283f) return __int_as_float(0x7f800000);
+    if (x < -87.33654f) return 0.0f;
+    const float kf = rintf(x * 1.44269504f), p = exp_reduced(x, kf);
     const int k = (int)kf;  // -126 .. 128
     // one exact scaling by 2^k where 2^k is a float (k <= 127); k = 128 in
     // two halves.  Either way the only rounding is that of the final product.
     if (k <= 127) return p * __int_as_float((k + 127) << 23);
     return (p * __int_as_float((64 + 127) << 23)) * __int_as_float((k - 64 + 127) << 23);
+}
+__device__ __forceinline__ float pvr_expf(float x) {
+    if (!(fabsf(x) <= 87.0f)) return exp_edges(x);
+    const float t = __fadd_rn(__fmul_rn(x, 1.44269504f), 12582912.0f);  // 1.5 * 2^23 + k
+    return __fmul_rn(exp_reduced(x, __fadd_rn(t, -12582912.0f)),
+                     __int_as_float((__float_as_int(t) << 23) + 0x3f800000));
 }
 
 // The fast arithmetic's two special functions, each one hardware
@@ -86,6 +98,20 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
     asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// 1 / sqrt(x) rounded once, for x > 0.  Between 2^-100 and 2^100: with y the
+// hardware's approximation (2^-22.9) and e = 1 - x y^2 to twice the precision
+// by FMAs, y (1 + e/2 + 3 e^2/8) is within 2^-45 of the root before its one
+// rounding, and equals __frsqrt_rn for every float there (tests): 28 -> 11
+// issue cycles per warp.
+__device__ __forceinline__ float rsqrt_rn(float x) {
+    if (!(x >= 7.888609e-31f && x <= 1.2676506e30f)) return __frsqrt_rn(x);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float h = __fmul_rn(x, y), l = fmaf(x, y, -h);
+    const float e = fmaf(-l, y, fmaf(-h, y, 1.0f));
+    return fmaf(y, fmaf(__fmul_rn(e, 0.375f), e, __fmul_rn(e, 0.5f)), y);
 }
 
 // Ray of pixel (px, py), py counted from the bottom row: vertex-stage uv at

@@ -93,6 +93,23 @@ def _check_inputs(volume, lut, normals):
         raise ValueError("volume, lut and normals must be on one device")
 
 
+_WORKSPACE_BYTES = {}  # scene sizes -> (forward and table backward, voxel backward)
+
+
+def _workspace_bytes(c):
+    """The workspaces' sizes of a scene (pvr_diff_workspace): they depend on
+    its sizes alone."""
+    key = (c.d, c.h, c.w, c.normals is None, c.width, c.height, c.n_views)
+    got = _WORKSPACE_BYTES.get(key)
+    if got is None:
+        n, n_vol = ctypes.c_longlong(0), ctypes.c_longlong(0)
+        check(_lib().pvr_diff_workspace(ctypes.byref(c), ctypes.byref(n), ctypes.byref(n_vol)))
+        if len(_WORKSPACE_BYTES) >= 256:
+            _WORKSPACE_BYTES.clear()
+        got = _WORKSPACE_BYTES[key] = (n.value, n_vol.value)
+    return got
+
+
 def _workspace(nbytes: int, device):
     """Scratch tensor in which a call packs the scene's texels, or None where
     that does not pay (0 bytes) or the memory is not there (the call then
@@ -122,14 +139,13 @@ def _march_function():
             steps = torch.empty((v, h, w), dtype=torch.int32, device=volume.device)
             c = scene.c_scene(volume, lut, normals)
             stream = torch.cuda.current_stream(volume.device).cuda_stream
-            n, n_vol = ctypes.c_longlong(0), ctypes.c_longlong(0)
-            check(_lib().pvr_diff_workspace(ctypes.byref(c), ctypes.byref(n), ctypes.byref(n_vol)))
-            ws = _workspace(n.value, volume.device)
+            nbytes = _workspace_bytes(c)
+            ws = _workspace(nbytes[0], volume.device)
             check(_lib().pvr_diff_forward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), ws[1], ws[2],
                                              stream))
             # the scene as it was rendered; the backward puts its own tensors' addresses in
             ctx.scene, ctx.c = scene, c
-            ctx.workspace_bytes = (n.value, n_vol.value)
+            ctx.workspace_bytes = nbytes
             ctx.save_for_backward(volume, lut, normals, image, steps)
             ctx.mark_non_differentiable(steps)
             return image, steps
