@@ -280,7 +280,7 @@ __device__ __forceinline__ bool brick_clear(const MarchFrame &f, float2 m, const
 template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST, int LERP, bool PACKED>
 __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, const float4 *lut,
                                           const int *prefix, float2 &acc_rg, float2 &acc_ba,
-                                          unsigned &n_inbox, unsigned &n_shaded) {
+                                          unsigned &n_skipped, unsigned &n_shaded) {
     constexpr int B = 1 << LOG2B, ROW = brick_apron(LOG2B), SLICE = ROW * ROW;
     constexpr int RECS = brick_records(LOG2B);
     const MarchFrame &f = job.f;
@@ -315,7 +315,6 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
                                txy.y <= 1.0f && tz >= 0.0f && tz <= 1.0f;
             if (valid) {
                 entered = true;
-                ++n_inbox;
                 // texel coordinate u = t*size - 0.5, lower texel k = floor(u)
                 const float2 sxy = PACKED ? __fmul2_rn(txy, fext_xy)
                                           : make_float2(__fmul_rn(txy.x, f.fext[0]), __fmul_rn(txy.y, f.fext[1]));
@@ -339,6 +338,8 @@ __device__ __forceinline__ void march_ray(const JobDesc &job, int px, int py, co
                     composite<FAST>(shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST, LERP>(
                                         f, bp + j, __fadd_rn(ux, -flx), __fadd_rn(uy, -fly), __fadd_rn(uz, -flz), lut),
                                     acc_rg, acc_ba);
+                } else {
+                    ++n_skipped;
                 }
             } else {
                 const bool never = entered || (txy.x < 0.0f && dxy.x <= 0.0f) ||
@@ -403,11 +404,11 @@ __device__ __forceinline__ void march_tile(const JobDesc &job, int px, int py, c
                                            const int *prefix, int lane) {
     const bool in_image = px < job.f.width && py < job.f.height;
     float2 acc_rg = make_float2(0.0f, 0.0f), acc_ba = make_float2(0.0f, 0.0f);
-    unsigned n_inbox = 0, n_shaded = 0;
+    unsigned n_skipped = 0, n_shaded = 0;
     if (in_image)
         march_ray<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, LERP, PACKED>(job, px, py, lut, prefix, acc_rg,
-                                                                                 acc_ba, n_inbox, n_shaded);
-    store_pixel(job, px, py, in_image, acc_rg, acc_ba, n_inbox, n_shaded, lane);
+                                                                                 acc_ba, n_skipped, n_shaded);
+    store_pixel(job, px, py, in_image, acc_rg, acc_ba, n_shaded + n_skipped, n_shaded, lane);
 }
 
 // Persistent batch kernel of one variant: normals or not, LUT staged in

@@ -138,7 +138,7 @@ def _march_function():
             image = torch.empty((v, h, w, 4), dtype=torch.float32, device=volume.device)
             steps = torch.empty((v, h, w), dtype=torch.int32, device=volume.device)
             c = scene.c_scene(volume, lut, normals)
-            stream = torch.cuda.current_stream(volume.device).cuda_stream
+            stream = torch.cuda.current_stream(volume.get_device()).cuda_stream
             nbytes = _workspace_bytes(c)
             ws = _workspace(nbytes[0], volume.device)
             check(_lib().pvr_diff_forward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), ws[1], ws[2],
@@ -161,7 +161,7 @@ def _march_function():
                 c = ctx.c
                 c.volume, c.lut = volume.data_ptr(), lut.data_ptr()
                 c.normals = normals.data_ptr() if normals is not None else None
-                stream = torch.cuda.current_stream(volume.device).cuda_stream
+                stream = torch.cuda.current_stream(volume.get_device()).cuda_stream
                 ws = _workspace(ctx.workspace_bytes[1 if need_vol else 0], volume.device)
                 check(_lib().pvr_diff_backward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(),
                                                   gimage.data_ptr(), glut.data_ptr() if glut is not None else None,
