@@ -400,6 +400,14 @@ __device__ __forceinline__ bool reduce_peers(unsigned peers, float v[8]) {
     return member;
 }
 
+// 1 / x for x in [2^-24, 2^126]: the hardware's approximation and one Newton
+// step by FMAs, within 0.51 ulp (1.4 % of a training step against the division).
+__device__ __forceinline__ float rcp_newton(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+
 // A warp's rays of one tile.  table: the warp's own LUT gradient (WARP_TABLE:
 // entry j of the LUT at table[j + 1], its apron below and above, written
 // without atomics: the lanes that write hold different entries), or the
@@ -429,7 +437,7 @@ __device__ __forceinline__ void backward_rays(const DiffParams &p, const MarchFr
             eval_sample<SOURCE>(p, f, t, lut, s);
             const float T = __fadd_rn(1.0f, -acc.w);
             composite(s, acc);
-            const float om = 1.0f - s.alpha, inv = om > 0.0f ? 1.0f / om : 0.0f;
+            const float om = 1.0f - s.alpha, inv = om > 0.0f ? rcp_newton(om) : 0.0f;
             const float cr = s.light * s.r, cg = s.light * s.g, cb = s.light * s.b;
             // T * (c - radiance behind) and T * (1 - alpha behind)
             const float br = (out.x - acc.x) * inv, bg = (out.y - acc.y) * inv, bb = (out.z - acc.z) * inv;
