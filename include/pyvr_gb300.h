@@ -373,13 +373,14 @@ int pvr_diff_backward(const pvr_diff_scene *scene, const float *d_image, const i
  * of a backward with d_grad_volume.  The scratch holds
  * nothing between calls, must be 16-byte aligned, and may be given back to
  * its owner's stream-ordered pool once the call has returned.  With NULL, or
- * fewer bytes, the calls are those above. */
+ * fewer bytes, the calls are those above.  overwrite != 0: the gradients are
+ * written instead of added to. */
 int pvr_diff_workspace(const pvr_diff_scene *scene, long long *bytes, long long *bytes_volume_gradient);
 int pvr_diff_forward_ws(const pvr_diff_scene *scene, float *d_image, int *d_steps, void *workspace,
                         long long workspace_bytes, void *stream);
 int pvr_diff_backward_ws(const pvr_diff_scene *scene, const float *d_image, const int *d_steps,
-                         const float *d_grad_image, float *d_grad_lut, float *d_grad_volume, void *workspace,
-                         long long workspace_bytes, void *stream);
+                         const float *d_grad_image, float *d_grad_lut, float *d_grad_volume, int overwrite,
+                         void *workspace, long long workspace_bytes, void *stream);
 
 /* ---- Serving runtime (no counterpart in the reference) -----------------
  * Continuous batching of render requests over resident volumes and LUTs on

@@ -154,7 +154,7 @@ SIGNATURES = {
     "pvr_diff_backward": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _VP]),
     "pvr_diff_workspace": (_I, [_VP, ctypes.POINTER(_LL), ctypes.POINTER(_LL)]),
     "pvr_diff_forward_ws": (_I, [_VP, _VP, _VP, _VP, _LL, _VP]),
-    "pvr_diff_backward_ws": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _LL, _VP]),
+    "pvr_diff_backward_ws": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _I, _VP, _LL, _VP]),
     "pvr_camera_spherical": (_I, [_FP, ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                   _FP, _FP, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                   ctypes.c_double, _FP, _FP, _FP]),

@@ -118,13 +118,16 @@ __host__ __device__ inline long long packed_texels(const int ext[3], bool normal
     return (long long)(ext[0] + 2) * (ext[1] + (normals ? 2 : 1)) * (ext[2] + (normals ? 2 : 1));
 }
 
-// Also clears the first nquads gradient quads (never more than the texels).
+// Also clears the first nquads gradient quads (never more than the texels)
+// and the first nglut floats of the LUT gradient.
 template <int SOURCE>
 __global__ void pack_kernel(const float *__restrict__ vol, const float *__restrict__ nrm, int ex, int ey, int ez,
-                            float4 *__restrict__ out, float4 *__restrict__ gquads, int nquads) {
+                            float4 *__restrict__ out, float4 *__restrict__ gquads, int nquads,
+                            float *__restrict__ glut, int nglut) {
     const int ny = ey + (SOURCE == kPackedNormals ? 2 : 1), nz = ez + (SOURCE == kPackedNormals ? 2 : 1);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = (ex + 2) * ny * nz;
+    for (int k = i; k < nglut; k += gridDim.x * blockDim.x) glut[k] = 0.0f;
     if (i >= total) return;
     if (i < nquads) gquads[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int z = i % nz, y = (i / nz) % ny, x = min(max(i / (nz * ny) - 1, 0), ex - 1);
@@ -141,7 +144,8 @@ __global__ void pack_kernel(const float *__restrict__ vol, const float *__restri
 
 // dL/dvoxel from the quads: voxel (x, y, z) is the lower and the upper corner
 // of two quad indices per axis, and of one more at each clamped face.
-__global__ void unpack_grad_kernel(const float4 *__restrict__ quads, int ex, int ey, int ez, float *__restrict__ gvol) {
+__global__ void unpack_grad_kernel(const float4 *__restrict__ quads, int ex, int ey, int ez, bool overwrite,
+                                   float *__restrict__ gvol) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ex * ey * ez) return;
     const int z = i % ez, y = (i / ez) % ey, x = i / (ez * ey);
@@ -159,7 +163,7 @@ __global__ void unpack_grad_kernel(const float4 *__restrict__ quads, int ex, int
                        (yu && zu ? q.w : 0.0f);
             }
     }
-    gvol[i] += sum;
+    gvol[i] = overwrite ? sum : gvol[i] + sum;
 }
 
 __device__ __forceinline__ int texel(const DiffParams &p, int x, int y, int z) {
@@ -623,16 +627,18 @@ int check_workspace(void *ws, long long bytes) {
 
 // Packs the scene's texels into the workspace where that pays and fits, and
 // (volume_gradient) clears the gradient quads behind them: where the march
-// then reads and adds.
+// then reads and adds.  clear_lut: a LUT gradient to clear as well, or null.
 struct Packed {
     int source = kLinear;
     const float4 *texels = nullptr;
     float4 *gquads = nullptr;
 };
-cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, void *ws, long long bytes, cudaStream_t st,
-                       Packed &out) {
+cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, float *clear_lut, void *ws, long long bytes,
+                       cudaStream_t st, Packed &out) {
     const long long need = packed_bytes(s, s->normals != nullptr), more = packed_bytes(s, false);
-    if (!ws || need == 0 || bytes < need) return cudaSuccess;
+    const int nglut = clear_lut ? 4 * s->lut_size : 0;
+    if (!ws || need == 0 || bytes < need)
+        return nglut ? cudaMemsetAsync(clear_lut, 0, nglut * sizeof(float), st) : cudaSuccess;
     float4 *texels = static_cast<float4 *>(ws);
     const int total = (int)(need / (long long)sizeof(float4)), blocks = (total + 255) / 256;
     out.source = s->normals ? kPackedNormals : kPackedQuads;
@@ -644,10 +650,10 @@ cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, void *ws, 
     }
     if (s->normals)
         pack_kernel<kPackedNormals><<<blocks, 256, 0, st>>>(s->volume, s->normals, s->w, s->h, s->d, texels,
-                                                            out.gquads, nquads);
+                                                            out.gquads, nquads, clear_lut, nglut);
     else
         pack_kernel<kPackedQuads><<<blocks, 256, 0, st>>>(s->volume, nullptr, s->w, s->h, s->d, texels, out.gquads,
-                                                          nquads);
+                                                          nquads, clear_lut, nglut);
     return cudaGetLastError();
 }
 
@@ -690,7 +696,7 @@ extern "C" int pvr_diff_forward_ws(const pvr_diff_scene *s, float *d_image, int 
         const int nv = std::min(pvr::kDiffMaxViews, s->n_views - v0);
         pvr::DiffParams p;
         if (int rc = pvr::build_params(s, v0, nv, p)) return rc;
-        if (v0 == 0) PVR_CUDA(pvr::pack_scene(s, false, workspace, workspace_bytes, st, packed));
+        if (v0 == 0) PVR_CUDA(pvr::pack_scene(s, false, nullptr, workspace, workspace_bytes, st, packed));
         p.texels = packed.texels;
         p.image = reinterpret_cast<float4 *>(d_image) + v0 * frame;
         p.steps = d_steps + v0 * frame;
@@ -707,7 +713,7 @@ extern "C" int pvr_diff_forward(const pvr_diff_scene *s, float *d_image, int *d_
 }
 
 extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_image, const int *d_steps,
-                                    const float *d_grad_image, float *d_grad_lut, float *d_grad_volume,
+                                    const float *d_grad_image, float *d_grad_lut, float *d_grad_volume, int overwrite,
                                     void *workspace, long long workspace_bytes, void *stream) {
     if (int rc = pvr::check_scene(s)) return rc;
     if (!d_image || !d_steps || !d_grad_image) return fail(PVR_ERR_VALUE, "image / steps / gradient buffer is NULL");
@@ -729,7 +735,10 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
         pvr::DiffParams p;
         if (int rc = pvr::build_params(s, v0, nv, p)) return rc;
         if (v0 == 0) {
-            PVR_CUDA(pvr::pack_scene(s, d_grad_volume != nullptr, workspace, workspace_bytes, st, packed));
+            PVR_CUDA(pvr::pack_scene(s, d_grad_volume != nullptr, overwrite ? d_grad_lut : nullptr, workspace,
+                                     workspace_bytes, st, packed));
+            if (overwrite && d_grad_volume && !packed.gquads)
+                PVR_CUDA(cudaMemsetAsync(d_grad_volume, 0, (size_t)s->d * s->h * s->w * sizeof(float), st));
             kernel = warp_table ? pvr::backward_kernel<true>(packed.source) : pvr::backward_kernel<false>(packed.source);
             // more than 48 KB of dynamic shared memory (set on the current device)
             if (smem > 48 * 1024)
@@ -751,7 +760,8 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
     }
     if (packed.gquads) {
         const int voxels = s->d * s->h * s->w;
-        pvr::unpack_grad_kernel<<<(voxels + 255) / 256, 256, 0, st>>>(packed.gquads, s->w, s->h, s->d, d_grad_volume);
+        pvr::unpack_grad_kernel<<<(voxels + 255) / 256, 256, 0, st>>>(packed.gquads, s->w, s->h, s->d, overwrite != 0,
+                                                                        d_grad_volume);
         PVR_CUDA(cudaGetLastError());
     }
     return PVR_OK;
@@ -760,5 +770,5 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
 extern "C" int pvr_diff_backward(const pvr_diff_scene *s, const float *d_image, const int *d_steps,
                                  const float *d_grad_image, float *d_grad_lut, float *d_grad_volume,
                                  void *stream) {
-    return pvr_diff_backward_ws(s, d_image, d_steps, d_grad_image, d_grad_lut, d_grad_volume, nullptr, 0, stream);
+    return pvr_diff_backward_ws(s, d_image, d_steps, d_grad_image, d_grad_lut, d_grad_volume, 0, nullptr, 0, stream);
 }

@@ -145,6 +145,8 @@ def _march_function():
                                              stream))
             # the scene as it was rendered; the backward puts its own tensors' addresses in
             ctx.scene, ctx.c = scene, c
+            # no zeros in the place of a gradient of `steps` (or of an unused image)
+            ctx.set_materialize_grads(False)
             ctx.workspace_bytes = nbytes
             ctx.save_for_backward(volume, lut, normals, image, steps)
             ctx.mark_non_differentiable(steps)
@@ -154,8 +156,11 @@ def _march_function():
         def backward(ctx, gimage, _gsteps):
             volume, lut, normals, image, steps = ctx.saved_tensors
             need_vol, need_lut = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-            gvol = torch.zeros_like(volume) if need_vol else None
-            glut = torch.zeros_like(lut) if need_lut else None
+            if gimage is None:
+                return (torch.zeros_like(volume) if need_vol else None, torch.zeros_like(lut) if need_lut else None,
+                        None, None)
+            gvol = torch.empty_like(volume) if need_vol else None
+            glut = torch.empty_like(lut) if need_lut else None
             if need_vol or need_lut:
                 gimage = gimage.contiguous()
                 c = ctx.c
@@ -165,7 +170,7 @@ def _march_function():
                 ws = _workspace(ctx.workspace_bytes[1 if need_vol else 0], volume.device)
                 check(_lib().pvr_diff_backward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(),
                                                   gimage.data_ptr(), glut.data_ptr() if glut is not None else None,
-                                                  gvol.data_ptr() if gvol is not None else None, ws[1], ws[2],
+                                                  gvol.data_ptr() if gvol is not None else None, 1, ws[1], ws[2],
                                                   stream))
             return gvol, glut, None, None
 
