@@ -160,13 +160,13 @@ static int layout_bricks(pvr_volume *v, cudaStream_t st, bool half, int bx0, int
 // as the texels they and their normals read have arrived, while the next
 // slab is on its way: a large volume is ready shortly after its last byte
 // (512^3 float16 from page-locked memory: upload 1.29 ms, then layout 0.56 ms:
-// 1.93 -> 1.50 ms; uint8 1.18 -> 0.84 ms).  Slabs of 16 MB and more, at most 8: a slab's copy
-// (80 us) then outweighs its launch, and the last slab's layout, which
-// nothing hides, stays an eighth of the whole.
+// 1.93 -> 1.48 ms; uint8 1.18 -> 0.83 ms).  Slabs of 8 MB on average, at most
+// 12 (their copies outweigh their launches), and thinner towards the end: the
+// last slab's layout is hidden by nothing (8 equal ones: 1.51 ms).
 static int upload_and_layout(pvr_volume *v, const char *data, cudaStream_t st, bool half) {
     const int ext = v->geo.ext[0], B = 1 << v->log2b;
     const size_t per_x = v->vol_bytes / (size_t)ext;
-    const int slabs = (int)std::min<size_t>(8, v->vol_bytes >> 24);
+    const int slabs = (int)std::min<size_t>(12, v->vol_bytes >> 23);
     cudaStream_t up = nullptr;
     cudaEvent_t arrived = nullptr;
     int lo = 0, hi = 0;
@@ -179,7 +179,7 @@ static int upload_and_layout(pvr_volume *v, const char *data, cudaStream_t st, b
     int rc = PVR_OK, x0 = 0, b0 = 0;
     for (int i = 1; i <= slabs && e == cudaSuccess && rc == PVR_OK; ++i) {
         // brick b reads texels up to (b + 1) * B (its apron's neighbour)
-        const int b1 = i == slabs ? v->geo.nb[0] : (int)((long long)v->geo.nb[0] * i / slabs);
+        const int b1 = i == slabs ? v->geo.nb[0] : (int)((long long)v->geo.nb[0] * i * (2 * slabs - i) / (slabs * slabs));
         const int x1 = i == slabs ? ext : std::min(ext, b1 * B + 1);
         if (x1 > x0)
             e = cudaMemcpyAsync((char *)v->d_vol + x0 * per_x, data + x0 * per_x, (size_t)(x1 - x0) * per_x,
