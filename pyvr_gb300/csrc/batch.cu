@@ -170,6 +170,22 @@ int build_graph(Slot &s, const LaunchKey &key, void **args) {
     return PVR_OK;
 }
 
+// Threads of a block of the single kernel, one per pixel of the tuning's tile
+// or of half of it: 128 for half records with normals, which are bound by
+// issue and at 512^2 by how the last blocks fall (1024 tiles on 760 slots), 256
+// else (float records share the lines of a tile: 128 threads 339 / 490 / 584 us
+// against 333 / 494 / 575).  Tables of 513 to 2048 entries keep 256 threads:
+// twice the blocks would stage them twice per SM.  Device us of half records,
+// 512^2 and 1024^2 balanced, 128 against 256 threads: 256^3 with 256 entries
+// 225, 537 / 232, 541, with 512 entries 226, 538 / 246, 557, with 1024 entries
+// 318, 602 / 252, 563, with 4096 (not staged) 240, 541 / 263, 553; 512^3 with
+// 256 entries 309, 612 / 330, 638, with 1024 entries 637, 866 / 355, 668.
+int single_threads(const pvr_volume &v, int lut_size) {
+    const bool half_tile = v.compact && v.normals_mode != PVR_NORMALS_NONE &&
+                           (lut_size <= 512 || lut_size > pvr::kMaxSmemLut);
+    return half_tile ? pvr::kBatchThreads / 2 : pvr::kBatchThreads;
+}
+
 // Lanes per ray of a single render that has the chip to itself: 4 or 2 where
 // all blocks of that kernel are resident at once (its launch bounds: 5 per SM
 // for half records, 4 for float ones), else 1.  Device us with 1 / 2 / 4 lanes,
@@ -210,8 +226,10 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
         // uses no work counter); the slot's event tracks it like a batch
         pvr::SingleParams &sp = b->single;
         const int lanes = b->split ? split_lanes(jobs[0].width, jobs[0].height, b->sms, jobs[0].volume->compact) : 1;
-        const int tile_w = lanes > 1 ? pvr::split_tile_w(lanes) : b->tuning.tile_w;
-        const int tile_h = lanes > 1 ? pvr::split_tile_h(lanes) : b->tuning.tile_h;
+        const int threads = lanes > 1 ? pvr::kBatchThreads : single_threads(*jobs[0].volume, max_lut);
+        int tile_w = lanes > 1 ? pvr::split_tile_w(lanes) : b->tuning.tile_w;
+        int tile_h = lanes > 1 ? pvr::split_tile_h(lanes) : b->tuning.tile_h;
+        if (threads < pvr::kBatchThreads) (tile_h > 4 ? tile_h : tile_w) /= 2;  // half the tuning's tile
         if (int rc = pvr::fill_job(jobs[0], tile_w, tile_h, fast, sp.job)) return rc;
         sp.tile_w = tile_w;
         sp.tile_h = tile_h;
@@ -225,7 +243,7 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
         void *args[] = {&sp};
         PVR_CUDA(cudaLaunchKernel(lanes > 1 ? pvr::split_kernel(log2b, lanes, variant)
                                             : pvr::single_kernel(log2b, b->tuning, variant), dim3((unsigned)tiles),
-                                  dim3(pvr::kBatchThreads), args, smem ? pvr::batch_smem_bytes(lut_smem) : 0,
+                                  dim3(threads), args, smem ? pvr::batch_smem_bytes(lut_smem) : 0,
                                   st));
         PVR_CUDA(cudaEventRecord(s.done, st));
         s.pending = true;

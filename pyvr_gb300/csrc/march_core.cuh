@@ -69,19 +69,22 @@ __device__ __forceinline__ float2 half_pair(uint32_t b) {
 }
 
 // How the lerps of a sample's records are written: the same two roundings per
-// lerp and lane in each.  Packed: two lanes per instruction.  Scalar: fewer
-// register pairs, for the kernel that has 40 registers.  Mixed: the first
+// lerp and lane in each.  Packed: two lanes per instruction.  Mixed: the first
 // lerp's difference b - a takes b as a half (one instruction of a half and a
-// float), so that only a is converted.  Measured per kernel, us (seeds of
-// the single and batch cases): half records at 40 registers packed 80.5 /
-// 135.6 / 143, scalar 76.3 / 131.5 / 136, mixed 94 / 141 / 160 (spills);
-// batches at 48 and 64 registers packed 1498 / 1526 / 1689, mixed 1441 / 1459
-// / 1638.
-enum LerpForm { kLerpPacked = 0, kLerpScalar = 1, kLerpMixed = 2 };
+// float), so that only a is converted.  MixedScalar: the same, one lane per
+// instruction, which needs no register pairs.  Half records in the single
+// kernel (us, three 512^2 orbit frames of 16^3 bricks / 1024^2 of 512^3):
+// scalar without the mixed difference at 40 registers 74 / 128 / 142 / 676,
+// MixedScalar at 40 (it spills) 77 / 139 / 156 / 686, at 48 79 / 119 / 130 /
+// 636, packed Mixed at 48 (spills) 82 / 130 / 135 / 655.  The split kernel at
+// 48: packed (spills) 123 / 291, MixedScalar 113 / 286 (192^2, 256^2 of 512^3).
+// The batch kernels at 48: packed 1498, Mixed 1441; later Mixed 1390,
+// MixedScalar 1440.
+enum LerpForm { kLerpPacked = 0, kLerpMixed = 1, kLerpMixedScalar = 2 };
 
 template <int LERP>
 __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float t) {
-    if (LERP == kLerpScalar) return make_float2(lerp_tex(a.x, b.x, t), lerp_tex(a.y, b.y, t));
+    if (LERP == kLerpMixedScalar) return make_float2(lerp_tex(a.x, b.x, t), lerp_tex(a.y, b.y, t));
     return lerp_tex2(a, b, t);
 }
 template <int LERP>
@@ -101,9 +104,11 @@ __device__ __forceinline__ float4 lerp_rec(float4 a, float4 b, float t) { return
 template <int LERP>
 __device__ __forceinline__ float4 lerp_rec(uint2 a, uint2 b, float t) {
     const float2 a0 = half_pair(a.x), a1 = half_pair(a.y);
-    if (LERP == kLerpMixed) {
+    if (LERP != kLerpPacked) {
         const float2 d0 = make_float2(sub_half(b.x, a0.x), sub_half(b.x >> 16, a0.y));
         const float2 d1 = make_float2(sub_half(b.y, a1.x), sub_half(b.y >> 16, a1.y));
+        if (LERP == kLerpMixedScalar)
+            return make_float4(fmaf(t, d0.x, a0.x), fmaf(t, d0.y, a0.y), fmaf(t, d1.x, a1.x), fmaf(t, d1.y, a1.y));
         const float2 x = __ffma2_rn(dup2(t), d0, a0), y = __ffma2_rn(dup2(t), d1, a1);
         return make_float4(x.x, x.y, y.x, y.y);
     }
@@ -466,11 +471,11 @@ march_batch_kernel(const __grid_constant__ BatchParams p) {
 // is the parameter block itself (static offsets), as in a plain frame kernel.
 // One instantiation per variant (normals, LUT in shared memory, half
 // records, arithmetic), chosen on the host: each gets its own register
-// allocation.  SMEM_LUT requires job.f.lut_size <= p.lut_smem_entries.  Half
-// records need 16 fewer registers for a sample's 8 records: those variants
-// run 6 blocks per SM (40 registers) instead of 5 (48).
+// allocation.  SMEM_LUT requires job.f.lut_size <= p.lut_smem_entries.  All
+// normals variants have 48 registers and 40 warps per SM; half records mostly
+// in blocks of 128 threads on half a tile (single_threads in batch.cu).
 template <int LOG2B, int UNROLL, bool NORMALS, bool SMEM_LUT, bool COMPACT, bool FAST>
-__global__ void __launch_bounds__(kBatchThreads, NORMALS ? (COMPACT ? 6 : 5) : 6)
+__global__ void __launch_bounds__(kBatchThreads, NORMALS ? 5 : 6)
 march_single_kernel(const __grid_constant__ SingleParams p) {
     extern __shared__ float4 s_dyn[];
     float4 *s_lut = s_dyn;
@@ -485,7 +490,7 @@ march_single_kernel(const __grid_constant__ SingleParams p) {
     const int t = blockIdx.x;
     const int px = (t % job.tiles_x) * p.tile_w + (warp % warps_x) * 8 + lane_x(lane);
     const int py = (t / job.tiles_x) * p.tile_h + (warp / warps_x) * 4 + lane_y(lane);
-    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, COMPACT ? kLerpScalar : kLerpPacked, true>(
+    march_tile<LOG2B, UNROLL, NORMALS, SMEM_LUT, COMPACT, FAST, COMPACT ? kLerpMixedScalar : kLerpPacked, true>(
         job, px, py, SMEM_LUT ? s_lut + 1 : job.lut, SMEM_LUT ? s_prefix : job.prefix, lane);
 }
 
@@ -572,7 +577,8 @@ march_split_kernel(const __grid_constant__ SingleParams p) {
             }
             if (!clear) {
                 const int j = (k[0] & (B - 1)) * SLICE + (k[1] & (B - 1)) * ROW + (k[2] & (B - 1));
-                s = shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST, kLerpPacked>(f, bp + j, fr[0], fr[1], fr[2], lut);
+                s = shade_sample<LOG2B, NORMALS, SMEM_LUT, FAST, COMPACT ? kLerpMixedScalar : kLerpPacked>(
+                    f, bp + j, fr[0], fr[1], fr[2], lut);
                 shaded = true;
             }
         }

@@ -78,3 +78,42 @@ def test_split_march(normals, records, dtype, lut_size):
                     assert np.array_equal(a8.reshape(o8.shape), o8) and an[0] == on
                     assert np.array_equal(af.reshape(of.shape).view(np.uint32), of.view(np.uint32))
     dv.close()
+
+
+# half a tile per block for half records, with tables that are staged (to 512
+# entries), staged with whole tiles (to 2048) and read from global memory
+@pytest.mark.parametrize("lut_size", [1, 512, 513, 2048, 2049])
+@pytest.mark.parametrize("tile_w,tile_h", [(16, 16), (64, 4), (8, 32)])
+def test_half_tiles(lut_size, tile_w, tile_h):
+    from pyvr_gb300 import OpacityTransferFunction
+    from pyvr_gb300.batch import (BatchRenderer, DeviceLUT, DeviceVolume, RenderJob, Tuning, arithmetic,
+                                  get_compact_records, set_compact_records)
+    vol = Volume(data=W.to_storage(W.value_noise((40, 40, 40), 6), "u8"), min_bounds=np.full(3, -1.0, np.float32),
+                 max_bounds=np.full(3, 1.0, np.float32))
+    prev = get_compact_records()
+    set_compact_records("half_normals")
+    try:
+        dv = DeviceVolume(vol, value_scale=1.0 / 255.0, normals="device", brick_log2=3)
+    finally:
+        set_compact_records(prev)
+    rgba = np.random.default_rng(lut_size).random((lut_size, 4)).astype(np.float32) * np.float32(0.4)
+    lut = DeviceLUT(rgba=rgba)
+    cam, light = Camera.from_spherical(np.zeros(3, np.float32), 0.7, 0.3, 0.0, 3.0), Light.directional([1, -1, 0], 0.2, 0.8)
+    for w, h in ((417, 331), (1029, 129)):  # more pixels than several lanes per ray take
+        for mode in ("exact", "fast"):
+            out = []
+            for n in (1, 2):  # alone, and as a job of the batch kernel
+                o8 = [torch.zeros(w * h * 4, dtype=torch.uint8, device="cuda") for _ in range(n)]
+                of = [torch.zeros(w * h * 4, dtype=torch.float32, device="cuda") for _ in range(n)]
+                c = torch.zeros((n, 2), dtype=torch.int64, device="cuda")
+                br = BatchRenderer(capacity=2, slots=1, tuning=Tuning(tile_w=tile_w, tile_h=tile_h, brick_log2=3))
+                torch.cuda.synchronize()
+                with arithmetic(mode):
+                    br.render([RenderJob(dv, lut, cam, light, RenderConfig.fast(), w, h, o8[k], of[k], c[k])
+                               for k in range(n)])
+                br.synchronize()
+                br.close()
+                out.append((o8[0].cpu().numpy(), of[0].cpu().numpy().view(np.uint32), c[0].tolist()))
+            assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]), (w, h, mode)
+            assert out[0][2] == out[1][2] and out[0][2][1] > 0, (w, h, mode)
+    dv.close()
