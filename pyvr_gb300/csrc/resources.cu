@@ -210,7 +210,7 @@ static void layout_queued(pvr_volume *v, cudaStream_t st, bool half) {
                        (v->dtype == PVR_F16 && v->normals_mode == PVR_NORMALS_DEVICE);
 }
 
-// Records, brick table and value ranges of a volume (once per volume).
+// Records, brick slots and value ranges of a volume (once per volume).
 int ensure_volume_layout(pvr_volume *v, cudaStream_t st) {
     if (v->layout_ready) return PVR_OK;
     bool half = false;
