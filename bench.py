@@ -61,16 +61,16 @@ NOMINAL_RATE = 400.0
 # (272^3-397^3) and of a 512^3 catalog, the upper end of the serving range
 # (profiles/march_single_kernel_serving_mix.md), and the plain 256^3 1024^2
 # high_quality frames (profiles/march_single_kernel_256cube_1024px.md)
-SERVING_WARP_INSTR_PER_SAMPLE = 7.51
-SERVING_DRAM_BYTES_PER_SAMPLE = 8.31
-SERVING_512_WARP_INSTR_PER_SAMPLE = 7.82
-SERVING_512_DRAM_BYTES_PER_SAMPLE = 23.4
-PLAIN_WARP_INSTR_PER_SAMPLE = 6.68
-PLAIN_DRAM_BYTES_PER_SAMPLE = 0.80
+SERVING_WARP_INSTR_PER_SAMPLE = 7.74
+SERVING_DRAM_BYTES_PER_SAMPLE = 8.14
+SERVING_512_WARP_INSTR_PER_SAMPLE = 8.04
+SERVING_512_DRAM_BYTES_PER_SAMPLE = 22.9
+PLAIN_WARP_INSTR_PER_SAMPLE = 6.78
+PLAIN_DRAM_BYTES_PER_SAMPLE = 0.78
 # ... and of the persistent batch kernel on the 64 uneven renders
 # (profiles/march_batch_kernel_batching64.md)
-BATCH_WARP_INSTR_PER_SAMPLE = 7.20
-BATCH_DRAM_BYTES_PER_SAMPLE = 1.20
+BATCH_WARP_INSTR_PER_SAMPLE = 6.84
+BATCH_DRAM_BYTES_PER_SAMPLE = 1.19
 P99_MS = 20.0
 # the requests whose latency the p99 bound applies to: the 512^2 frames
 # (orbit re-renders, TF edits, and the renders of newly loaded volumes, the
@@ -499,8 +499,8 @@ def serving_section(args, torch):
                                        per_sample_512cube={"warp_instr": SERVING_512_WARP_INSTR_PER_SAMPLE,
                                                            "dram_bytes": SERVING_512_DRAM_BYTES_PER_SAMPLE,
                                                            "note": "the same kernel on 512^3 uint8 volumes "
-                                                                   "(upper end of the catalog): bound by L1 "
-                                                                   "traffic (84 %) and gather latency"},
+                                                                   "(upper end of the catalog): bound by the "
+                                                                   "latency of gathers that miss L1"},
                                        profile="profiles/march_single_kernel_serving_mix.md"),
                clocks=clk, h2d=h2d / args.steps, d2h=d2h / args.steps, setup_s=setup_s, pool=pool,
                loads=srv["loads"], evictions=srv["evictions"],
