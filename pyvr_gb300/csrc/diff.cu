@@ -663,6 +663,13 @@ const void *forward_kernel(int source) {
                                     : (const void *)diff_forward_kernel<kLinear>;
 }
 
+// Dynamic shared memory of the backward kernel: the LUT and its apron, and
+// with a LUT gradient as many entries per warp, or once more for the block.
+int backward_smem(int lut_size, bool lut_gradient) {
+    const int tables = !lut_gradient ? 0 : lut_size <= kWarpTableLut ? kDiffThreads / 32 : 1;
+    return (lut_size + 2) * (int)sizeof(float4) * (1 + tables);
+}
+
 template <bool WARP_TABLE>
 const void *backward_kernel(int source) {
     return source == kPackedNormals ? (const void *)diff_backward_kernel<kPackedNormals, WARP_TABLE>
@@ -724,8 +731,7 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
     PVR_CUDA(cudaGetDevice(&device));
     PVR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const bool warp_table = s->lut_size <= pvr::kWarpTableLut;
-    const size_t rows = (size_t)s->lut_size + 2;
-    const size_t smem = rows * sizeof(float4) * (d_grad_lut ? (warp_table ? 1 + pvr::kDiffThreads / 32 : 2) : 1);
+    const int smem = pvr::backward_smem(s->lut_size, d_grad_lut != nullptr);
     int per_sm = 0;
     pvr::Packed packed;
     const void *kernel = nullptr;
@@ -740,9 +746,14 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
             if (overwrite && d_grad_volume && !packed.gquads)
                 PVR_CUDA(cudaMemsetAsync(d_grad_volume, 0, (size_t)s->d * s->h * s->w * sizeof(float), st));
             kernel = warp_table ? pvr::backward_kernel<true>(packed.source) : pvr::backward_kernel<false>(packed.source);
-            // more than 48 KB of dynamic shared memory (set on the current device)
+            // more than 48 KB of dynamic shared memory: the limit belongs to the
+            // kernel on the current device, not to this call, so every call sets
+            // the most that any table takes (a smaller limit would refuse the
+            // launch of another thread's larger table)
             if (smem > 48 * 1024)
-                PVR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                PVR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              warp_table ? pvr::backward_smem(pvr::kWarpTableLut, true)
+                                                         : pvr::backward_smem(pvr::kDiffMaxLut, true)));
             PVR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, pvr::kDiffThreads, smem));
             per_sm = std::max(1, per_sm);
         }

@@ -1,0 +1,53 @@
+"""The differentiable march called from several threads at once: the C entry
+points take no handle, so calls with different table sizes may overlap."""
+
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+from pyvr_gb300 import Camera, Light, RenderConfig, _native
+from pyvr_gb300.diff import DiffScene
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _scene():
+    cam = Camera.from_spherical(np.zeros(3, np.float32), 0.3, 0.4, 0.0, 3.0)
+    return DiffScene([cam], Light.directional([1, -1, 0], 0.2, 0.8), RenderConfig.fast(), 16, 16)
+
+
+# two per-warp tables of more than 48 KB, and two per-block ones
+@pytest.mark.parametrize("sizes", [(512, 400), (2048, 1600)])
+def test_backward_calls_of_different_table_sizes(sizes):
+    lib, scene, errors = _native.load(), _scene(), []
+
+    def work(n):
+        torch.cuda.set_device(0)
+        vol, lut = torch.rand(8, 8, 8, device="cuda"), torch.rand(n, 4, device="cuda") * 0.1
+        image = torch.empty((1, 16, 16, 4), device="cuda")
+        steps = torch.empty((1, 16, 16), dtype=torch.int32, device="cuda")
+        g, glut = torch.ones_like(image), torch.zeros_like(lut)
+        torch.cuda.synchronize()
+        stream = torch.cuda.Stream()
+        c = scene.c_scene(vol, lut)
+        rc = lib.pvr_diff_forward(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), stream.cuda_stream)
+        for k in range(4000):
+            if rc:
+                errors.append((n, lib.pvr_last_error()))
+                break
+            rc = lib.pvr_diff_backward(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), g.data_ptr(),
+                                       glut.data_ptr(), None, stream.cuda_stream)
+            if k % 64 == 0:
+                stream.synchronize()
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
