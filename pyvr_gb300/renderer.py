@@ -23,11 +23,12 @@ from .lighting import Light
 
 
 # a bytes object of n uninitialised bytes, and its address: an image is copied
-# from the device into the object it is returned in
-_bytes_new = ctypes.pythonapi.PyBytes_FromStringAndSize
-_bytes_new.restype, _bytes_new.argtypes = ctypes.py_object, [ctypes.c_char_p, ctypes.c_ssize_t]
-_bytes_address = ctypes.pythonapi.PyBytes_AsString
-_bytes_address.restype, _bytes_address.argtypes = ctypes.c_void_p, [ctypes.py_object]
+# from the device into the object it is returned in.  Function objects of
+# their own: those of ctypes.pythonapi, and their prototypes, are the whole
+# process's
+_bytes_new = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_char_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
+_bytes_address = ctypes.PYFUNCTYPE(ctypes.c_void_p, ctypes.py_object)(("PyBytes_AsString", ctypes.pythonapi))
 
 _F3, _F16 = ctypes.c_float * 3, ctypes.c_float * 16
 
