@@ -162,9 +162,11 @@ __device__ __forceinline__ float2 half_root(float2 x) {
     const float2 s = __fmul2_rn(x, r);
     return __ffma2_rn(__ffma2_rn(__fmul2_rn(s, both(-1.0f)), s, x), __fmul2_rn(r, both(0.5f)), s);
 }
+// The remainder enters negated, q n - g times -r: as g - q n times r (one
+// product fewer) a g of -0 gave +0, where the division gives -0.
 __device__ __forceinline__ float2 half_quotient(float2 g, float2 n, float2 r) {
     const float2 q = __fmul2_rn(g, r);
-    return __ffma2_rn(__ffma2_rn(__fmul2_rn(q, both(-1.0f)), n, g), r, q);
+    return __ffma2_rn(__ffma2_rn(q, n, __fmul2_rn(g, both(-1.0f))), __fmul2_rn(r, both(-1.0f)), q);
 }
 __device__ __forceinline__ float2 f16_square_sum(__half2 g0, __half2 g1, __half2 g2) {
     const float2 s = __fadd2_rn(__fadd2_rn(__half22float2(__hmul2(g0, g0)), __half22float2(__hmul2(g1, g1))),
