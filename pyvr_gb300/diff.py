@@ -143,7 +143,7 @@ def _march_function():
             ws = _workspace(nbytes[0], volume.device)
             check(_lib().pvr_diff_forward_ws(ctypes.byref(c), image.data_ptr(), steps.data_ptr(), ws[1], ws[2],
                                              stream))
-            # the scene as it was rendered; the backward puts its own tensors' addresses in
+            # the scene as it was rendered; a backward puts its own tensors' addresses into a copy
             ctx.scene, ctx.c = scene, c
             # no zeros in the place of a gradient of `steps` (or of an unused image)
             ctx.set_materialize_grads(False)
@@ -163,7 +163,8 @@ def _march_function():
             glut = torch.empty_like(lut) if need_lut else None
             if need_vol or need_lut:
                 gimage = gimage.contiguous()
-                c = ctx.c
+                # a copy: two threads may run this backward at once (retain_graph)
+                c = _native.PvrDiffScene.from_buffer_copy(ctx.c)
                 c.volume, c.lut = volume.data_ptr(), lut.data_ptr()
                 c.normals = normals.data_ptr() if normals is not None else None
                 stream = torch.cuda.current_stream(volume.get_device()).cuda_stream

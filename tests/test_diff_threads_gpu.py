@@ -51,3 +51,21 @@ def test_backward_calls_of_different_table_sizes(sizes):
     for t in threads:
         t.join()
     assert not errors
+
+
+def test_backward_leaves_the_saved_scene_alone():
+    # saved-tensor hooks give every backward tensors of its own; their
+    # addresses must not reach another backward of the same graph
+    from pyvr_gb300.diff import render_views
+    vol = torch.rand(8, 8, 8, device="cuda").requires_grad_()
+    lut = (torch.rand(64, 4, device="cuda") * 0.1).requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t.clone()):
+        image = render_views(vol, lut, _scene())
+    saved = bytes(image.grad_fn.c)
+    image.backward(torch.ones_like(image), retain_graph=True)
+    first = lut.grad.clone(), vol.grad.clone()
+    assert bytes(image.grad_fn.c) == saved
+    image.backward(torch.ones_like(image))
+    # up to the order of the float sums
+    for got, one in ((lut.grad, first[0]), (vol.grad, first[1])):
+        assert float((got - 2 * one).abs().max()) <= 1e-4 * float(one.abs().max())
