@@ -47,9 +47,11 @@ def _norm(v: np.ndarray):
 
 
 def _cross(a: np.ndarray, b: np.ndarray) -> np.ndarray:
-    """np.cross of two 3-vectors of one float type: the same products and
-    differences in that type, as scalars (a frame's camera took most of its
-    time in np.cross's setup: 87 -> 38 us per set_camera)."""
+    """np.cross of two 3-vectors: the same products and differences in their
+    common type, as scalars (a frame's camera took most of its time in
+    np.cross's setup: 87 -> 38 us per set_camera).  Sequences are taken too (a
+    Camera subclass may give its vectors as lists)."""
+    a, b = np.asarray(a), np.asarray(b)
     if a.dtype == np.float64 and b.dtype == np.float64:
         a, b, dtype = a.tolist(), b.tolist(), np.float64
     else:
