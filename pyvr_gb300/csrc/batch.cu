@@ -104,7 +104,6 @@ struct pvr_batch {
     std::unique_ptr<pvr::BatchParams> params;  // host staging of one launch's job table
     pvr::SingleParams single;                  // ... of a one-job launch
     bool split = true;  // small single renders may take several lanes per ray
-    bool tuned = false;  // pvr_batch_set_tuning was called: its blocks per SM hold
 };
 
 using pvr::fail;
@@ -274,9 +273,7 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
     if (!(variant & pvr::kSingleSmemLut)) lut_smem = 0;  // the LUTs are read from global memory
     p.lut_smem_entries = lut_smem;
     p.work = s.d_work;
-    // without a tuning of the caller's, as many persistent blocks as fit: 5 per
-    // SM for half records against 4, 32 uneven renders 1437 -> 1400 us
-    int per_sm = b->tuned ? b->tuning.blocks_per_sm : 0;
+    int per_sm = b->tuning.blocks_per_sm;
     const int fit = pvr::max_batch_blocks_per_sm(log2b, b->tuning, lut_smem, variant);
     if (per_sm <= 0 || per_sm > fit) per_sm = std::max(1, fit);
     LaunchKey key;
@@ -348,7 +345,6 @@ int pvr_batch_set_tuning(pvr_batch *b, const pvr_tuning *tuning) {
         return fail(PVR_ERR_VALUE, "tuning: tile_w%%8==0, tile_h%%4==0, tile_w*tile_h==256, "
                                    "steps_per_iter in {1,4}, blocks_per_sm in 0..16");
     b->tuning = t;
-    b->tuned = true;
     return PVR_OK;
 }
 

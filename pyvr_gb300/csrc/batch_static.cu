@@ -226,7 +226,7 @@ extern "C" int pvr_batch_render_static(const pvr_job *jobs, int n, const pvr_tun
             if (!(v & pvr::kSingleSmemLut)) lut_smem = 0;  // the LUTs are read from global memory
             p.lut_smem_entries = lut_smem;
             p.work = counters + c;
-            int per_sm = tuning ? t.blocks_per_sm : 0;  // without a tuning, as many as fit
+            int per_sm = t.blocks_per_sm;
             const int fit = pvr::max_batch_blocks_per_sm(log2b, t, lut_smem, v);
             if (per_sm <= 0 || per_sm > fit) per_sm = std::max(1, fit);
             void *args[] = {&p};
