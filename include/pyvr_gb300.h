@@ -291,7 +291,14 @@ typedef struct {
 /* Launch shape of the persistent batch kernel: tile_w x tile_h pixels per
  * 256-thread block (tile_w a multiple of 8, tile_h of 4, product 256),
  * march steps per loop iteration (1 or 4), persistent blocks per SM
- * (0 = as many as fit). */
+ * (0 = as many as fit).  A call with one render has one block per tile; half
+ * records may take half of the tile per block.  The default, {16, 16, 1, 0},
+ * leaves the launch of one small render (up to about 280^2 pixels) to the
+ * library, which gives each ray 2 or 4 lanes: 1.7 times as fast on average,
+ * alone and on up to 4 streams.  Where 8 streams keep the device full of such
+ * renders, one lane per ray has more throughput (256^2 frames, 62 against
+ * 69 us each; without normals 22 against 30): any other shape is taken as it
+ * is, for instance {16, 16, 1, 4}. */
 typedef struct pvr_tuning_s {
     int tile_w, tile_h, steps_per_iter, blocks_per_sm;
 } pvr_tuning;

@@ -108,6 +108,38 @@ struct pvr_batch {
 
 using pvr::fail;
 
+namespace pvr {
+
+// Lanes per ray of a single render that has the chip to itself: 4 or 2 where
+// all blocks of that kernel are resident at once (its launch bounds: 5 per SM
+// for half records, 4 for float ones), else 1.  Device us with 1 / 2 / 4 lanes,
+// 256^3 uint8 in float records, 384^3 float16 in half records (balanced) and
+// 64^3 float32 (high quality):
+//   192^2   59.8 / 40.2 / 38.7    79.5 / 41.1 / 34.9    63.6 / 44.2 / 36.8
+//   256^2   64.3 / 55.1 / 59.1    84.0 / 53.7 / 52.4    65.0 / 57.7 / 53.5
+//   384^2   78.5 / 78.2 / 87.5    93.9 / 83.1 / 81.2    87.4 / 85.5 / 89.5
+//   512^2  102.7 / 103.7 / 130   103.5 / 104.5 / 117   122.7 / 125.7 / 142
+// A second wave of blocks loses where most rays hit the box (153x938: 46.0 us
+// with 1 lane, 54.2 with 2); in one wave 102 random frames of up to 10^5 pixels
+// were 1.5 times as fast on average, the worst 0.93 (16.6 -> 17.7 us).
+int split_lanes(int width, int height, int sms, bool compact) {
+    for (int lanes = 4; lanes >= 2; lanes /= 2) {
+        const int tw = pvr::split_tile_w(lanes), th = pvr::split_tile_h(lanes);
+        const long long tiles = (long long)((width + tw - 1) / tw) * ((height + th - 1) / th);
+        if (tiles <= (long long)sms * pvr::split_blocks_per_sm(compact)) return lanes;
+    }
+    return 1;
+}
+
+// The default shape leaves the launch to the library; any other is the caller's
+// and is taken as it is, with one lane per ray.
+int render_lanes(const pvr_batch *b, const pvr_job &j) {
+    if (!b->split || !(b->tuning == Tuning())) return 1;
+    return split_lanes(j.width, j.height, b->sms, j.volume->compact);
+}
+
+}  // namespace pvr
+
 namespace {
 
 void destroy_slot(Slot &s) {
@@ -185,27 +217,6 @@ int single_threads(const pvr_volume &v, int lut_size) {
     return half_tile ? pvr::kBatchThreads / 2 : pvr::kBatchThreads;
 }
 
-// Lanes per ray of a single render that has the chip to itself: 4 or 2 where
-// all blocks of that kernel are resident at once (its launch bounds: 5 per SM
-// for half records, 4 for float ones), else 1.  Device us with 1 / 2 / 4 lanes,
-// 256^3 uint8 in float records, 384^3 float16 in half records (balanced) and
-// 64^3 float32 (high quality):
-//   192^2   59.8 / 40.2 / 38.7    79.5 / 41.1 / 34.9    63.6 / 44.2 / 36.8
-//   256^2   64.3 / 55.1 / 59.1    84.0 / 53.7 / 52.4    65.0 / 57.7 / 53.5
-//   384^2   78.5 / 78.2 / 87.5    93.9 / 83.1 / 81.2    87.4 / 85.5 / 89.5
-//   512^2  102.7 / 103.7 / 130   103.5 / 104.5 / 117   122.7 / 125.7 / 142
-// A second wave of blocks loses where most rays hit the box (153x938: 46.0 us
-// with 1 lane, 54.2 with 2); in one wave 102 random frames of up to 10^5 pixels
-// were 1.5 times as fast on average, the worst 0.93 (16.6 -> 17.7 us).
-int split_lanes(int width, int height, int sms, bool compact) {
-    for (int lanes = 4; lanes >= 2; lanes /= 2) {
-        const int tw = pvr::split_tile_w(lanes), th = pvr::split_tile_h(lanes);
-        const long long tiles = (long long)((width + tw - 1) / tw) * ((height + th - 1) / th);
-        if (tiles <= (long long)sms * pvr::split_blocks_per_sm(compact)) return lanes;
-    }
-    return 1;
-}
-
 // One launch over jobs[idx[0..n)] (jobs of one variant, at most
 // kMaxLaunchJobs).
 int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool fast, cudaStream_t st) {
@@ -224,7 +235,7 @@ int launch_chunk(pvr_batch *b, const pvr_job *all, const int *idx, int n, bool f
         // launched directly (its parameters are copied at the launch, and it
         // uses no work counter); the slot's event tracks it like a batch
         pvr::SingleParams &sp = b->single;
-        const int lanes = b->split ? split_lanes(jobs[0].width, jobs[0].height, b->sms, jobs[0].volume->compact) : 1;
+        const int lanes = pvr::render_lanes(b, jobs[0]);
         const int threads = lanes > 1 ? pvr::kBatchThreads : single_threads(*jobs[0].volume, max_lut);
         int tile_w = lanes > 1 ? pvr::split_tile_w(lanes) : b->tuning.tile_w;
         int tile_h = lanes > 1 ? pvr::split_tile_h(lanes) : b->tuning.tile_h;

@@ -105,6 +105,10 @@ struct Tuning {
     int tile_w = 16, tile_h = 16;
     int steps_per_iter = 1;
     int blocks_per_sm = 0;
+    bool operator==(const Tuning &o) const {
+        return tile_w == o.tile_w && tile_h == o.tile_h && steps_per_iter == o.steps_per_iter &&
+               blocks_per_sm == o.blocks_per_sm;
+    }
 };
 
 // March kernels (march_core.cuh), one instantiation per brick size and
@@ -119,9 +123,12 @@ const void *single_kernel(int log2b, const Tuning &t, int variant);
 // The kernel for one small render with 2 or 4 lanes per ray, and the pixels of
 // one of its blocks.
 const void *split_kernel(int log2b, int lanes, int variant);
-// Whether launches of this batch may use it: not beside others on the device,
-// where several lanes per ray cost throughput.
+// Whether launches of this batch may use it: not where others keep the device
+// full, where several lanes per ray cost throughput.
 void batch_allow_split(pvr_batch *b, bool allow);
+// Lanes per ray of a single render: by its size, and of a launcher (its shape).
+int split_lanes(int width, int height, int sms, bool compact);
+int render_lanes(const pvr_batch *b, const pvr_job &j);
 __host__ __device__ constexpr int split_blocks_per_sm(bool compact) { return compact ? 5 : 4; }
 __host__ __device__ constexpr int split_tile_w(int) { return 8; }
 __host__ __device__ constexpr int split_tile_h(int lanes) { return 32 / lanes; }

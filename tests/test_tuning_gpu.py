@@ -23,3 +23,24 @@ def test_reported_default_is_what_runs():
     default = Tuning()
     assert (t.tile_w, t.tile_h, t.steps_per_iter, t.blocks_per_sm) == (
         default.tile_w, default.tile_h, default.steps_per_iter, default.blocks_per_sm) == (16, 16, 1, 0)
+
+
+def test_shapes_of_the_caller_keep_one_lane_per_ray():
+    import numpy as np
+
+    from pyvr_gb300 import Camera, Light, RenderConfig, Volume
+    from pyvr_gb300.batch import BatchRenderer, DeviceLUT, DeviceVolume, RenderJob, Tuning, make_job_struct
+    lanes = getattr(_native.load(), "_ZN3pvr12render_lanesEPK9pvr_batchRK7pvr_job")
+    lanes.argtypes, lanes.restype = [ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int
+    dv = DeviceVolume(Volume(data=np.ones((9, 9, 9), np.float32)), normals="none")
+    lut = DeviceLUT(rgba=np.full((4, 4), 0.1, np.float32))
+    cam = Camera.from_spherical(np.zeros(3, np.float32), 0.7, 0.3, 0.0, 3.0)
+    job = make_job_struct(RenderJob(dv, lut, cam, Light.directional([1, -1, 0], 0.2, 0.8), RenderConfig.fast(), 64, 48))
+    br = BatchRenderer(capacity=1, slots=1)
+    assert lanes(br.handle, ctypes.byref(job)) == 4
+    for t, want in ((Tuning(), 4), (Tuning(8, 32, 1, 0), 1), (Tuning(16, 16, 4, 0), 1), (Tuning(16, 16, 1, 4), 1),
+                    (Tuning(), 4)):
+        br.set_tuning(t)
+        assert lanes(br.handle, ctypes.byref(job)) == want, t
+    br.close()
+    dv.close()
