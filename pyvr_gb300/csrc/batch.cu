@@ -120,13 +120,21 @@ namespace pvr {
 //   384^2   78.5 / 78.2 / 87.5    93.9 / 83.1 / 81.2    87.4 / 85.5 / 89.5
 //   512^2  102.7 / 103.7 / 130   103.5 / 104.5 / 117   122.7 / 125.7 / 142
 // A second wave of blocks loses where most rays hit the box (153x938: 46.0 us
-// with 1 lane, 54.2 with 2); in one wave 102 random frames of up to 10^5 pixels
-// were 1.5 times as fast on average, the worst 0.93 (16.6 -> 17.7 us).
-int split_lanes(int width, int height, int sms, bool compact) {
+// with 1 lane, 54.2 with 2).  Near the full wave 2 lanes gain least: random
+// frames of 40^3 to 320^3 texels, time with 1 lane / with 2, by the share of
+// the resident blocks that a frame takes (mean, worst, frames that lose 2 %):
+//   float records        0.5-0.8: 1.43, 0.99, 0 of 178   0.8-1: 1.35, 0.94, 5 of 95
+//   half, 2^21 texels up 0.5-0.8: 1.32, 1.04, 0 of 110   0.8-1: 1.21, 0.95, 5 of 59
+//   half, fewer          0.5-0.8: 1.20, 0.92, 12 of 102  0.8-1: 1.15, 0.82, 20 of 56
+// Half records of a small volume mostly come from L1, and one lane per ray
+// is then bound by issue, not latency: the last case takes 1 lane.  4 lanes
+// at 0.75 to 1: 1.73, worst 1.05 of 60.
+int split_lanes(int width, int height, int sms, bool compact, long long texels) {
     for (int lanes = 4; lanes >= 2; lanes /= 2) {
         const int tw = pvr::split_tile_w(lanes), th = pvr::split_tile_h(lanes);
         const long long tiles = (long long)((width + tw - 1) / tw) * ((height + th - 1) / th);
-        if (tiles <= (long long)sms * pvr::split_blocks_per_sm(compact)) return lanes;
+        const bool small = lanes == 2 && compact && texels < (1 << 21);
+        if (tiles <= (long long)sms * (small ? 4 : pvr::split_blocks_per_sm(compact))) return lanes;
     }
     return 1;
 }
@@ -135,7 +143,8 @@ int split_lanes(int width, int height, int sms, bool compact) {
 // and is taken as it is, with one lane per ray.
 int render_lanes(const pvr_batch *b, const pvr_job &j) {
     if (!b->split || !(b->tuning == Tuning())) return 1;
-    return split_lanes(j.width, j.height, b->sms, j.volume->compact);
+    const int *d = j.volume->dims;
+    return split_lanes(j.width, j.height, b->sms, j.volume->compact, (long long)d[0] * d[1] * d[2]);
 }
 
 }  // namespace pvr

@@ -127,7 +127,7 @@ const void *split_kernel(int log2b, int lanes, int variant);
 // full, where several lanes per ray cost throughput.
 void batch_allow_split(pvr_batch *b, bool allow);
 // Lanes per ray of a single render: by its size, and of a launcher (its shape).
-int split_lanes(int width, int height, int sms, bool compact);
+int split_lanes(int width, int height, int sms, bool compact, long long texels);
 int render_lanes(const pvr_batch *b, const pvr_job &j);
 __host__ __device__ constexpr int split_blocks_per_sm(bool compact) { return compact ? 5 : 4; }
 __host__ __device__ constexpr int split_tile_w(int) { return 8; }
