@@ -23,7 +23,10 @@ reported beside it.  The roofline is the batch march kernel's
 (event-timed launches in the timed steps; bytes = 8 voxel texels in the
 stored type + 8 float32x3 normal texels per shaded in-box sample).
 
-Nested sections: "plain" (the per-frame renderer on 256^3 value noise in
+The last line of stdout is the headline's JSON object (under 4 KB: logs keep
+tails); before it one JSON object with the details goes to stderr.
+
+Details: "plain" (the per-frame renderer on 256^3 value noise in
 u8/f16/f32, 16 orbit cameras, 1024^2, high_quality; one step = 48 frames),
 "batching_c3" (64 uneven renders per persistent launch with the autotuner's
 settings) and "differentiation" (TF recovery with the hand-written backward).
@@ -129,6 +132,21 @@ def parse_args():
 def dist_env():
     return (int(os.environ.get("RANK", "0")), int(os.environ.get("WORLD_SIZE", "1")),
             int(os.environ.get("LOCAL_RANK", "0")))
+
+
+# the keys of the headline's line; everything else is details
+HEADLINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+                 "vs_baseline", "dtype", "data", "config", "clocks", "e2e", "gpu_launches", "cpu_baseline",
+                 "serial_per_frame", "roofline_issue_frac", "roofline_dram_frac", "sustained_offered", "p99_all_ms",
+                 "p50_ms", "p99_ms", "server_over_serial")
+
+
+def print_result(result):
+    """The details as one JSON object on stderr, then the headline's line on
+    stdout."""
+    details = {k: v for k, v in result.items() if k not in HEADLINE_KEYS}
+    print(json.dumps(details), file=sys.stderr, flush=True)
+    print(json.dumps({k: result[k] for k in HEADLINE_KEYS}), flush=True)
 
 
 def measured_peaks():
@@ -1100,8 +1118,6 @@ def run_ours(args):
     if rank == 0:
         srv = s["server"]
         att, satt = s["attempts"]["server"][-1], s["attempts"]["serial"][-1]
-        # nested sections first, the headline's own keys last: the end of
-        # the line is what a log tail keeps
         line = {"plain": plain, "batching_c3": batching, "differentiation": diff, "loaders": loaders,
                 "nominal_400": s["nominal"],
                 "probes": {"server": s["probes_server"], "serial": s["probes_serial"]},
@@ -1137,7 +1153,7 @@ def run_ours(args):
                 "sustained_offered": s["rate_server"], "p99_all_ms": srv.get("p99_ms"),
                 "p50_ms": s["server_frames"].get("p50_ms"), "p99_ms": s["server_frames"].get("p99_ms"),
                 "server_over_serial": value / serial_value if serial_value else None}
-        print(json.dumps(line))
+        print_result(line)
     if world > 1:
         torch.distributed.destroy_process_group()
 
