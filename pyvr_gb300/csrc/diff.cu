@@ -404,14 +404,6 @@ __device__ __forceinline__ bool reduce_peers(unsigned peers, float v[8]) {
     return member;
 }
 
-// 1 / x for x in [2^-24, 2^126]: the hardware's approximation and one Newton
-// step by FMAs, within 0.51 ulp (1.4 % of a training step against the division).
-__device__ __forceinline__ float rcp_newton(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
-}
-
 // A warp's rays of one tile.  table: the warp's own LUT gradient (WARP_TABLE:
 // entry j of the LUT at table[j + 1], its apron below and above, written
 // without atomics: the lanes that write hold different entries), or the

@@ -114,6 +114,16 @@ __device__ __forceinline__ float rsqrt_rn(float x) {
     return fmaf(y, fmaf(__fmul_rn(e, 0.375f), e, __fmul_rn(e, 0.5f)), y);
 }
 
+// 1 / x for x in [2^-24, 2^126]: the hardware's approximation (2^-23) and one
+// Newton step by FMAs, which leaves 2^-46 before its rounding: within 0.51 ulp
+// (tests; 1.4 % of a training step against the division).  Beyond 2^126 it
+// gives 0 (NaN for infinity).
+__device__ __forceinline__ float rcp_newton(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+
 // Ray of pixel (px, py), py counted from the bottom row: vertex-stage uv at
 // the pixel centre (volume.vert.glsl:8), ray_direction (frag:47-54) and the
 // slab test (frag:56-68, 75-81).  Returns false for a miss.
