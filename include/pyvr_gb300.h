@@ -292,13 +292,14 @@ typedef struct {
  * 256-thread block (tile_w a multiple of 8, tile_h of 4, product 256),
  * march steps per loop iteration (1 or 4), persistent blocks per SM
  * (0 = as many as fit).  A call with one render has one block per tile; half
- * records may take half of the tile per block.  The default, {16, 16, 1, 0},
- * leaves the launch of one small render (up to about 280^2 pixels) to the
- * library, which gives each ray 2 or 4 lanes: 1.7 times as fast on average,
- * alone and on up to 4 streams.  Where 8 streams keep the device full of such
- * renders, one lane per ray has more throughput (256^2 frames, 62 against
- * 69 us each; without normals 22 against 30): any other shape is taken as it
- * is, for instance {16, 16, 1, 4}. */
+ * records may take half of the tile per block, and blocks per SM do not
+ * matter.  The default tile and steps, {16, 16, 1}, leave the launch of one
+ * small render (up to about 280^2 pixels) to the library, which gives each ray
+ * 2 or 4 lanes: 1.7 times as fast on average, alone and on up to 4 streams.
+ * Where 8 streams keep the device full of such renders, one lane per ray has
+ * more throughput (256^2 frames, 62 against 69 us each; without normals 22
+ * against 30): any other tile or steps are taken as they are, for instance
+ * {8, 32, 1, 0}. */
 typedef struct pvr_tuning_s {
     int tile_w, tile_h, steps_per_iter, blocks_per_sm;
 } pvr_tuning;

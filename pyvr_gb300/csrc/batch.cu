@@ -139,10 +139,13 @@ int split_lanes(int width, int height, int sms, bool compact, long long texels) 
     return 1;
 }
 
-// The default shape leaves the launch to the library; any other is the caller's
-// and is taken as it is, with one lane per ray.
+// The default tile and steps leave the launch to the library; any others are
+// the caller's and are taken as they are, with one lane per ray.  (Blocks per
+// SM are a batch's: a tuning that differs only there keeps the lanes, 64
+// single renders of 128^2 to 1024^2 with 5 per SM 4.7 against 5.4 ms.)
 int render_lanes(const pvr_batch *b, const pvr_job &j) {
-    if (!b->split || !(b->tuning == Tuning())) return 1;
+    const Tuning &t = b->tuning, d0;
+    if (!b->split || t.tile_w != d0.tile_w || t.tile_h != d0.tile_h || t.steps_per_iter != d0.steps_per_iter) return 1;
     const int *d = j.volume->dims;
     return split_lanes(j.width, j.height, b->sms, j.volume->compact, (long long)d[0] * d[1] * d[2]);
 }

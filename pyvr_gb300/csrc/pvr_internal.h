@@ -105,10 +105,6 @@ struct Tuning {
     int tile_w = 16, tile_h = 16;
     int steps_per_iter = 1;
     int blocks_per_sm = 0;
-    bool operator==(const Tuning &o) const {
-        return tile_w == o.tile_w && tile_h == o.tile_h && steps_per_iter == o.steps_per_iter &&
-               blocks_per_sm == o.blocks_per_sm;
-    }
 };
 
 // March kernels (march_core.cuh), one instantiation per brick size and

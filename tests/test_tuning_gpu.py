@@ -25,7 +25,7 @@ def test_reported_default_is_what_runs():
         default.tile_w, default.tile_h, default.steps_per_iter, default.blocks_per_sm) == (16, 16, 1, 0)
 
 
-def test_shapes_of_the_caller_keep_one_lane_per_ray():
+def test_tiles_and_steps_of_the_caller_keep_one_lane_per_ray():
     import numpy as np
 
     from pyvr_gb300 import Camera, Light, RenderConfig, Volume
@@ -38,8 +38,9 @@ def test_shapes_of_the_caller_keep_one_lane_per_ray():
     job = make_job_struct(RenderJob(dv, lut, cam, Light.directional([1, -1, 0], 0.2, 0.8), RenderConfig.fast(), 64, 48))
     br = BatchRenderer(capacity=1, slots=1)
     assert lanes(br.handle, ctypes.byref(job)) == 4
-    for t, want in ((Tuning(), 4), (Tuning(8, 32, 1, 0), 1), (Tuning(16, 16, 4, 0), 1), (Tuning(16, 16, 1, 4), 1),
-                    (Tuning(), 4)):
+    # blocks per SM are a batch's
+    for t, want in ((Tuning(), 4), (Tuning(8, 32, 1, 0), 1), (Tuning(16, 16, 4, 0), 1), (Tuning(64, 4, 1, 0), 1),
+                    (Tuning(16, 16, 1, 5), 4), (Tuning(), 4)):
         br.set_tuning(t)
         assert lanes(br.handle, ctypes.byref(job)) == want, t
     br.close()
