@@ -57,9 +57,11 @@ constexpr int kDiffMaxLut = 2048;   // LUT entries (shared-memory gradient)
 // larger ones one per block
 constexpr int kWarpTableLut = 512;
 
-// Where a sample's texels come from: the scene's arrays, or packed texels
-// with normals, or packed (y, z) quads of values.
-enum TexelSource { kLinear = 0, kPackedNormals = 1, kPackedQuads = 2 };
+// Where a sample's texels come from: the scene's arrays (8 or, with normals,
+// 32 scalar loads), or packed texels with normals, or packed (y, z) quads of
+// values.
+enum TexelSource { kLinear = 0, kLinearNormals = 1, kPackedNormals = 2, kPackedQuads = 3 };
+__host__ __device__ constexpr bool is_packed(int source) { return source >= kPackedNormals; }
 
 struct DiffParams {
     const float *vol;       // (D, H, W) C order: texel (x, y, z) at (x * H + y) * D + z
@@ -170,25 +172,27 @@ __device__ __forceinline__ int texel(const DiffParams &p, int x, int y, int z) {
     return (x * p.ext[1] + y) * p.ext[2] + z;
 }
 
-// value (and normal) at a sample, from the scene's own arrays
-__device__ __forceinline__ float tri(const float *v, const DiffParams &p, const Sample &s, int stride, int c) {
+// The 8 texels of a sample in the scene's own arrays; bits 2, 1 and 0 of the
+// index: upper x, y and z.
+struct Corners {
+    int i[8];
+};
+__device__ __forceinline__ Corners corners(const DiffParams &p, const Sample &s) {
     int lo[3], hi[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         lo[a] = max(s.k[a], 0);
         hi[a] = min(s.k[a] + 1, p.ext[a] - 1);
     }
-    const float v000 = __ldg(v + texel(p, lo[0], lo[1], lo[2]) * stride + c);
-    const float v001 = __ldg(v + texel(p, lo[0], lo[1], hi[2]) * stride + c);
-    const float v010 = __ldg(v + texel(p, lo[0], hi[1], lo[2]) * stride + c);
-    const float v011 = __ldg(v + texel(p, lo[0], hi[1], hi[2]) * stride + c);
-    const float v100 = __ldg(v + texel(p, hi[0], lo[1], lo[2]) * stride + c);
-    const float v101 = __ldg(v + texel(p, hi[0], lo[1], hi[2]) * stride + c);
-    const float v110 = __ldg(v + texel(p, hi[0], hi[1], lo[2]) * stride + c);
-    const float v111 = __ldg(v + texel(p, hi[0], hi[1], hi[2]) * stride + c);
-    const float c0 = lerp_tex(lerp_tex(v000, v001, s.fz), lerp_tex(v010, v011, s.fz), s.fy);
-    const float c1 = lerp_tex(lerp_tex(v100, v101, s.fz), lerp_tex(v110, v111, s.fz), s.fy);
-    return lerp_tex(c0, c1, s.fx);
+    Corners c;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c.i[k] = texel(p, k & 4 ? hi[0] : lo[0], k & 2 ? hi[1] : lo[1], k & 1 ? hi[2] : lo[2]);
+    return c;
+}
+
+__device__ __forceinline__ float lerp8(const float v[8], const Sample &s) {
+    return lerp_tex(lerp_tex(lerp_tex(v[0], v[1], s.fz), lerp_tex(v[2], v[3], s.fz), s.fy),
+                    lerp_tex(lerp_tex(v[4], v[5], s.fz), lerp_tex(v[6], v[7], s.fz), s.fy), s.fx);
 }
 
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
@@ -229,13 +233,21 @@ __device__ __forceinline__ float fetch(const DiffParams &p, const MarchFrame &f,
         const float2 y = lerp2(make_float2(z0.x, z1.x), make_float2(z0.y, z1.y), s.fy);
         density = __fmul_rn(lerp_tex(y.x, y.y, s.fx), f.value_scale);
     } else {
-        density = __fmul_rn(tri(p.vol, p, s, 1, 0), f.value_scale);
-        if (p.nrm) {
-            n[0] = tri(p.nrm, p, s, 3, 0);
-            n[1] = tri(p.nrm, p, s, 3, 1);
-            n[2] = tri(p.nrm, p, s, 3, 2);
-            return density;
+        const Corners c = corners(p, s);
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __ldg(p.vol + c.i[k]);
+        if (SOURCE == kLinearNormals) {
+            float m[3][8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) m[a][k] = __ldg(p.nrm + 3 * c.i[k] + a);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) n[a] = lerp8(m[a], s);
+            return __fmul_rn(lerp8(v, s), f.value_scale);
         }
+        density = __fmul_rn(lerp8(v, s), f.value_scale);
     }
     // the reference's unbound normal sampler reads the volume
     n[0] = density;
@@ -246,7 +258,9 @@ __device__ __forceinline__ float fetch(const DiffParams &p, const MarchFrame &f,
 
 // Everything one in-box sample computes (frag:93-110), with the renderer's
 // rounding.  lut: the table in shared memory with an apron entry at either
-// end (lut[-1] = lut[0], lut[size] = lut[size - 1]).
+// end (lut[-1] = lut[0], lut[size] = lut[size - 1]); for the scene's own arrays
+// the table itself, since scalar gathers need L1 more: staged, 2048 entries
+// took a 104^3 volume's forward from 65 to 72 us (48 registers) and 156 (40).
 template <int SOURCE>
 __device__ __forceinline__ void eval_sample(const DiffParams &p, const MarchFrame &f, const float t[3],
                                            const float4 *lut, Sample &s) {
@@ -266,8 +280,13 @@ __device__ __forceinline__ void eval_sample(const DiffParams &p, const MarchFram
     const float lfl = floorf(lu);
     s.la = __fadd_rn(lu, -lfl);
     s.j0 = (int)fminf(fmaxf(lfl, -1.0f), f.flut_max);  // NaN: -1
-    s.A = lut[s.j0];
-    s.B = lut[s.j0 + 1];
+    if (is_packed(SOURCE)) {
+        s.A = lut[s.j0];
+        s.B = lut[s.j0 + 1];
+    } else {
+        s.A = __ldg(lut + max(s.j0, 0));
+        s.B = __ldg(lut + min(s.j0 + 1, f.lut_size - 1));
+    }
     const float2 rg = lerp2(lo2(s.A), lo2(s.B), s.la), ba = lerp2(hi2(s.A), hi2(s.B), s.la);
     s.r = rg.x;
     s.g = rg.y;
@@ -310,13 +329,23 @@ __device__ __forceinline__ const float4 *stage_diff_lut(const DiffParams &p, flo
     return s_lut + 1;
 }
 
-// Dynamic shared memory: the LUT and its apron (lut_size + 2 entries).
+// Blocks per SM that the forward's registers allow (0: the compiler's choice):
+// the 32 loads of a sample of the scene's arrays with normals need 64
+// registers to be in flight together (220 random scenes against the scalar kernel before packing: 1.02 times as fast on average at 48, the worst
+// 0.78; 1.09 at 64, the worst 0.94).
+constexpr int forward_blocks(int source) { return source == kLinearNormals ? 4 : source == kLinear ? 5 : 0; }
+
+// Dynamic shared memory (packed sources): the LUT and its apron (lut_size + 2
+// entries).
 template <int SOURCE>
-__global__ void __launch_bounds__(kDiffThreads)
+__global__ void __launch_bounds__(kDiffThreads, forward_blocks(SOURCE))
 diff_forward_kernel(const __grid_constant__ DiffParams p) {
     extern __shared__ float4 s_dyn[];
-    const float4 *lut = stage_diff_lut(p, s_dyn);
-    __syncthreads();
+    const float4 *lut = p.lut;
+    if (is_packed(SOURCE)) {
+        lut = stage_diff_lut(p, s_dyn);
+        __syncthreads();
+    }
     const int per_view = p.tiles_x * p.tiles_y;
     const int view = blockIdx.x / per_view;
     const MarchFrame &f = p.f[view];
@@ -348,6 +377,8 @@ diff_forward_kernel(const __grid_constant__ DiffParams p) {
     p.steps[idx] = i;
 }
 
+// Adds a sample's voxel gradient (packed sources) to the quads, or without them
+// (too small a workspace) to the voxels.
 __device__ __forceinline__ void add_voxel_grad(const DiffParams &p, const Sample &s, float gd) {
     const float wx[2] = {1.0f - s.fx, s.fx}, wy[2] = {1.0f - s.fy, s.fy}, wz[2] = {1.0f - s.fz, s.fz};
     if (p.gquads) {
@@ -404,6 +435,30 @@ __device__ __forceinline__ bool reduce_peers(unsigned peers, float v[8]) {
     return member;
 }
 
+// Adds the warp's voxel gradients (gd of each lane, 0 for none; the scene's own
+// arrays as source) to the voxels.  All rays of a warp are at the same step, so neighbouring ones
+// mostly add to the same 8 voxels: lanes with the same ones sum first, or
+// their atomics queue up (36x47x28 voxels under a 91x634 image: 1395 -> 268 us).
+// All lanes of the warp call it.
+__device__ __forceinline__ void add_voxel_grads(const DiffParams &p, const Sample &s, float gd) {
+    const bool adds = gd != 0.0f;
+    if (!__any_sync(0xffffffffu, adds)) return;
+    unsigned key = 0xffffffffu - (threadIdx.x & 31);  // no peers
+    float v[8] = {};
+    if (adds) {
+        key = ((unsigned)(s.k[0] + 1) * (p.ext[1] + 1) + (s.k[1] + 1)) * (p.ext[2] + 1) + (s.k[2] + 1);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v[k] = gd * (k & 4 ? s.fx : 1.0f - s.fx) * (k & 2 ? s.fy : 1.0f - s.fy) * (k & 1 ? s.fz : 1.0f - s.fz);
+    }
+    if (reduce_peers(__match_any_sync(0xffffffffu, key), v) && adds) {
+        const Corners c = corners(p, s);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (v[k] != 0.0f) atomicAdd(p.gvol + c.i[k], v[k]);
+    }
+}
+
 // A warp's rays of one tile.  table: the warp's own LUT gradient (WARP_TABLE:
 // entry j of the LUT at table[j + 1], its apron below and above, written
 // without atomics: the lanes that write hold different entries), or the
@@ -427,9 +482,9 @@ __device__ __forceinline__ void backward_rays(const DiffParams &p, const MarchFr
         float t[3];
         const bool sampled = tex_coords(f, pos, t) && i < nsteps;
         unsigned key = 0xffff0000u | threadIdx.x;  // no peers
-        float v[8];
+        float v[8], gd = 0.0f;
+        Sample s;
         if (sampled) {
-            Sample s;
             eval_sample<SOURCE>(p, f, t, lut, s);
             const float T = __fadd_rn(1.0f, -acc.w);
             composite(s, acc);
@@ -447,14 +502,15 @@ __device__ __forceinline__ void backward_rays(const DiffParams &p, const MarchFr
             v[4] = w1 * dr; v[5] = w1 * dg; v[6] = w1 * db; v[7] = w1 * da;
             key = (unsigned)(s.j0 + 1);
             if (p.gvol) {
-                const float gd = (dr * (s.B.x - s.A.x) + dg * (s.B.y - s.A.y) + db * (s.B.z - s.A.z) +
-                                  da * (s.B.w - s.A.w)) * f.flut_size * f.value_scale;
-                if (gd != 0.0f) add_voxel_grad(p, s, gd);
+                gd = (dr * (s.B.x - s.A.x) + dg * (s.B.y - s.A.y) + db * (s.B.z - s.A.z) +
+                      da * (s.B.w - s.A.w)) * f.flut_size * f.value_scale;
+                if (is_packed(SOURCE) && gd != 0.0f) add_voxel_grad(p, s, gd);
             }
         } else {
 #pragma unroll
             for (int c = 0; c < 8; ++c) v[c] = 0.0f;
         }
+        if (!is_packed(SOURCE) && p.gvol) add_voxel_grads(p, s, gd);
 #pragma unroll
         for (int a = 0; a < 3; ++a) pos[a] = __fadd_rn(pos[a], d[a]);
         if (table) {
@@ -489,17 +545,17 @@ __device__ __forceinline__ void backward_rays(const DiffParams &p, const MarchFr
     }
 }
 
-// Persistent blocks over the tiles.  Dynamic shared memory: the LUT and its
-// apron, then (p.glut) the gradient tables: one of lut_size + 2 entries per
-// warp, or one channel-major table per block.
+// Persistent blocks over the tiles.  Dynamic shared memory: (packed sources)
+// the LUT and its apron, then (p.glut) the gradient tables: one of lut_size + 2
+// entries per warp, or one channel-major table per block.
 template <int SOURCE, bool WARP_TABLE>
 __global__ void __launch_bounds__(kDiffThreads)
 diff_backward_kernel(const __grid_constant__ DiffParams p) {
     extern __shared__ float4 s_dyn[];
     constexpr int kWarps = kDiffThreads / 32;
     const int size = p.f[0].lut_size, rows = size + 2;
-    const float4 *lut = stage_diff_lut(p, s_dyn);
-    float4 *tables = s_dyn + rows;
+    const float4 *lut = is_packed(SOURCE) ? stage_diff_lut(p, s_dyn) : p.lut;
+    float4 *tables = is_packed(SOURCE) ? s_dyn + rows : s_dyn;
     if (p.glut)
         for (int k = threadIdx.x; k < (WARP_TABLE ? kWarps * rows : size); k += kDiffThreads)
             tables[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -621,7 +677,7 @@ int check_workspace(void *ws, long long bytes) {
 // (volume_gradient) clears the gradient quads behind them: where the march
 // then reads and adds.  clear_lut: a LUT gradient to clear as well, or null.
 struct Packed {
-    int source = kLinear;
+    int source = kLinear;  // or kLinearNormals: set by pack_scene
     const float4 *texels = nullptr;
     float4 *gquads = nullptr;
 };
@@ -629,6 +685,7 @@ cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, float *cle
                        cudaStream_t st, Packed &out) {
     const long long need = packed_bytes(s, s->normals != nullptr), more = packed_bytes(s, false);
     const int nglut = clear_lut ? 4 * s->lut_size : 0;
+    out.source = s->normals ? kLinearNormals : kLinear;
     if (!ws || need == 0 || bytes < need)
         return nglut ? cudaMemsetAsync(clear_lut, 0, nglut * sizeof(float), st) : cudaSuccess;
     float4 *texels = static_cast<float4 *>(ws);
@@ -650,23 +707,29 @@ cudaError_t pack_scene(const pvr_diff_scene *s, bool volume_gradient, float *cle
 }
 
 const void *forward_kernel(int source) {
-    return source == kPackedNormals ? (const void *)diff_forward_kernel<kPackedNormals>
-           : source == kPackedQuads ? (const void *)diff_forward_kernel<kPackedQuads>
-                                    : (const void *)diff_forward_kernel<kLinear>;
+    switch (source) {
+    case kPackedNormals: return (const void *)diff_forward_kernel<kPackedNormals>;
+    case kPackedQuads: return (const void *)diff_forward_kernel<kPackedQuads>;
+    case kLinearNormals: return (const void *)diff_forward_kernel<kLinearNormals>;
+    default: return (const void *)diff_forward_kernel<kLinear>;
+    }
 }
 
-// Dynamic shared memory of the backward kernel: the LUT and its apron, and
-// with a LUT gradient as many entries per warp, or once more for the block.
-int backward_smem(int lut_size, bool lut_gradient) {
+// Dynamic shared memory of the backward kernel: for packed sources the LUT and
+// its apron, and with a LUT gradient as many entries per warp, or for the block.
+int backward_smem(int source, int lut_size, bool lut_gradient) {
     const int tables = !lut_gradient ? 0 : lut_size <= kWarpTableLut ? kDiffThreads / 32 : 1;
-    return (lut_size + 2) * (int)sizeof(float4) * (1 + tables);
+    return (lut_size + 2) * (int)sizeof(float4) * ((is_packed(source) ? 1 : 0) + tables);
 }
 
 template <bool WARP_TABLE>
 const void *backward_kernel(int source) {
-    return source == kPackedNormals ? (const void *)diff_backward_kernel<kPackedNormals, WARP_TABLE>
-           : source == kPackedQuads ? (const void *)diff_backward_kernel<kPackedQuads, WARP_TABLE>
-                                    : (const void *)diff_backward_kernel<kLinear, WARP_TABLE>;
+    switch (source) {
+    case kPackedNormals: return (const void *)diff_backward_kernel<kPackedNormals, WARP_TABLE>;
+    case kPackedQuads: return (const void *)diff_backward_kernel<kPackedQuads, WARP_TABLE>;
+    case kLinearNormals: return (const void *)diff_backward_kernel<kLinearNormals, WARP_TABLE>;
+    default: return (const void *)diff_backward_kernel<kLinear, WARP_TABLE>;
+    }
 }
 
 }  // namespace
@@ -702,7 +765,7 @@ extern "C" int pvr_diff_forward_ws(const pvr_diff_scene *s, float *d_image, int 
         const int blocks = p.tiles_x * p.tiles_y * nv;
         void *args[] = {&p};
         PVR_CUDA(cudaLaunchKernel(pvr::forward_kernel(packed.source), dim3(blocks), dim3(pvr::kDiffThreads), args,
-                                  (size_t)(s->lut_size + 2) * sizeof(float4), st));
+                                  pvr::is_packed(packed.source) ? (size_t)(s->lut_size + 2) * sizeof(float4) : 0, st));
     }
     return PVR_OK;
 }
@@ -723,8 +786,7 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
     PVR_CUDA(cudaGetDevice(&device));
     PVR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const bool warp_table = s->lut_size <= pvr::kWarpTableLut;
-    const int smem = pvr::backward_smem(s->lut_size, d_grad_lut != nullptr);
-    int per_sm = 0;
+    int per_sm = 0, smem = 0;
     pvr::Packed packed;
     const void *kernel = nullptr;
     const long long frame = (long long)s->width * s->height;
@@ -738,14 +800,14 @@ extern "C" int pvr_diff_backward_ws(const pvr_diff_scene *s, const float *d_imag
             if (overwrite && d_grad_volume && !packed.gquads)
                 PVR_CUDA(cudaMemsetAsync(d_grad_volume, 0, (size_t)s->d * s->h * s->w * sizeof(float), st));
             kernel = warp_table ? pvr::backward_kernel<true>(packed.source) : pvr::backward_kernel<false>(packed.source);
+            smem = pvr::backward_smem(packed.source, s->lut_size, d_grad_lut != nullptr);
             // more than 48 KB of dynamic shared memory: the limit belongs to the
             // kernel on the current device, not to this call, so every call sets
             // the most that any table takes (a smaller limit would refuse the
             // launch of another thread's larger table)
             if (smem > 48 * 1024)
                 PVR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              warp_table ? pvr::backward_smem(pvr::kWarpTableLut, true)
-                                                         : pvr::backward_smem(pvr::kDiffMaxLut, true)));
+                                              pvr::backward_smem(packed.source, warp_table ? pvr::kWarpTableLut : pvr::kDiffMaxLut, true)));
             PVR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, pvr::kDiffThreads, smem));
             per_sm = std::max(1, per_sm);
         }
