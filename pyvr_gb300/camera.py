@@ -49,9 +49,7 @@ def _norm(v: np.ndarray):
 def _cross(a: np.ndarray, b: np.ndarray) -> np.ndarray:
     """np.cross of two 3-vectors: the same products and differences in their
     common type, as scalars (a frame's camera took most of its time in
-    np.cross's setup: 87 -> 38 us per set_camera).  Sequences are taken too (a
-    Camera subclass may give its vectors as lists)."""
-    a, b = np.asarray(a), np.asarray(b)
+    np.cross's setup: 87 -> 38 us per set_camera)."""
     if a.dtype == np.float64 and b.dtype == np.float64:
         a, b, dtype = a.tolist(), b.tolist(), np.float64
     else:
@@ -238,7 +236,7 @@ class Camera:
         """get_view_matrix from already computed camera vectors."""
         fwd = self.target - position
         fwd = fwd / _norm(fwd)
-        right = _cross(fwd, up)
+        right = _cross(fwd, np.asarray(up))  # a subclass may give lists
         right = right / _norm(right)
         up_c = _cross(right, fwd)
         m = np.zeros((4, 4), dtype=np.float64)
