@@ -114,9 +114,10 @@ int pvr_render(pvr_renderer *r, uint8_t *out_rgba8, float *out_rgba32f);
 /* render() (renderer.py:209-219) into the handle's own page-locked RGBA8
  * image (width*height*4 bytes, allocated on first use): the image comes
  * back by DMA with no staging copy, and *rgba8 receives its address.  The
- * buffer stays valid, unchanged, until the next render call on the handle or
- * pvr_destroy; a binding copies it into the `bytes` it returns.  Synchronous;
- * the same image as pvr_render. */
+ * buffer stays valid, unchanged, until the next pvr_render_pinned on the handle
+ * or pvr_destroy.  Synchronous; the same image as pvr_render.  (A binding that
+ * returns bytes is faster with pvr_render into them: on the GB300's host link
+ * the copy into pageable memory takes no longer, and the second copy goes.) */
 int pvr_render_pinned(pvr_renderer *r, const uint8_t **rgba8);
 
 /* Same march into caller-owned DEVICE buffers on `stream` (NULL = the
@@ -376,8 +377,8 @@ int pvr_diff_backward(const pvr_diff_scene *scene, const float *d_image, const i
                       void *stream);
 
 /* The same two with device scratch of the caller's, in which the scene's texels
- * are packed for the march (and voxel gradients gathered): several times
- * faster.  pvr_diff_workspace gives the bytes that help (0: none do), and those
+ * are packed for the march (and voxel gradients gathered): 1.0 to 2.4 times as
+ * fast (with normals 1.3 on average, without 1.1).  pvr_diff_workspace gives the bytes that help (0: none do), and those
  * of a backward with d_grad_volume.  The scratch holds
  * nothing between calls, must be 16-byte aligned, and may be given back to
  * its owner's stream-ordered pool once the call has returned.  With NULL, or

@@ -35,9 +35,10 @@
 // a workspace (pvr_diff_workspace) each call first packs the volume into
 // 16-byte texels, which the march reads with 8 loads (value and normal of a
 // texel) or, without normals, 2 (the four (y, z) corners of a texel).
-// Measured on 128^3 with normals, 8 views of 512^2: forward 985 -> 515 us,
-// backward to the LUT 3250 -> 1020 us (with the front-to-back order), the packing 13 us of each; 72^3
-// without normals, 3 views of 251x197, backward to voxels and LUT 303 -> 110 us.
+// Measured on 128^3 with normals, 8 views of 512^2, from the scene's arrays and
+// walking backward -> now (the profile's launches): forward 985 -> 400 us,
+// backward to the LUT 3250 -> 820 us, the packing 13 us of each; 72^3 without
+// normals, 3 views of 251x197, backward to voxels and LUT 303 -> 110 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -54,7 +55,10 @@ constexpr int kDiffThreads = 256;   // 16 x 16 pixel tile; warps cover 8 x 4 pix
 constexpr int kDiffTile = 16;
 constexpr int kDiffMaxLut = 2048;   // LUT entries (shared-memory gradient)
 // LUTs up to this many entries get a gradient table per warp (8 KB each),
-// larger ones one per block
+// larger ones one per block, whose float atomics cost more than the L1 that
+// the tables take: 128^3 with normals, 8 views of 512^2, high opacity, backward
+// us with warp tables / one table, 272 entries 2568 / 3156, 384 2546 / 3076,
+// 512 2480 / 2925.  Three blocks per SM fit up to about 530 entries.
 constexpr int kWarpTableLut = 512;
 
 // Where a sample's texels come from: the scene's arrays (8 or, with normals,
@@ -331,8 +335,9 @@ __device__ __forceinline__ const float4 *stage_diff_lut(const DiffParams &p, flo
 
 // Blocks per SM that the forward's registers allow (0: the compiler's choice):
 // the 32 loads of a sample of the scene's arrays with normals need 64
-// registers to be in flight together (220 random scenes against the scalar kernel before packing: 1.02 times as fast on average at 48, the worst
-// 0.78; 1.09 at 64, the worst 0.94).
+// registers to be in flight together (113 random scenes against the kernel
+// before packing: at 48 registers 1.02 times as fast on average, the worst
+// 0.78; at 64 1.09, the worst 0.89).
 constexpr int forward_blocks(int source) { return source == kLinearNormals ? 4 : source == kLinear ? 5 : 0; }
 
 // Dynamic shared memory (packed sources): the LUT and its apron (lut_size + 2

@@ -275,8 +275,10 @@ __device__ __forceinline__ void write_range(float lo, float hi, uint4 *brick) {
 // of size (D,H,W) read through the z/y/x swizzle, volume.frag.glsl:90).
 // Measured: 512^3 in 33^3 bricks of 17^3 half records, float16 1720 -> 557 us,
 // uint8 1722 -> 457 us; 256^3 in bricks of 9^3 float records, uint8 338 -> 152 us,
-// float32 249 -> 121 us.  16^3 bricks: 4 blocks per SM (48 registers); at 3 (64
-// registers, float16 796 us) and 5 (32, spills, 744 us) it is slower.
+// float32 249 -> 121 us.  16^3 bricks: 4 blocks per SM (48 registers, with spills:
+// 64 bytes for float16, 168 for float32 with normals); 3 (64 registers) and 5
+// (32) are slower: 512^3 float16 557 us against 796 and 744, 200^3 float32 51
+// us against 59 with 3 (without normals 43 against 46).
 template <typename T, int LOG2B, typename Rec, bool NORMALS>
 __global__ void __launch_bounds__(BrickShape<LOG2B>::kThreads, LOG2B == 4 ? 4 : 1)
 build_walk_kernel(BrickGeometry g, const T *__restrict__ vol, int brick0, Rec *__restrict__ records,

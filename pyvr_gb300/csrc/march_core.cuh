@@ -1,17 +1,19 @@
-// The ray-march kernel: pyvr/shaders/volume.frag.glsl:main as CUDA, run as
-// a persistent kernel over a batch of renders.
+// The ray-march kernels: pyvr/shaders/volume.frag.glsl:main as CUDA, run as
+// a persistent kernel over a batch of renders, as a kernel of one render (one
+// block per tile), and as one of a small render with several lanes per ray.
 //
-// Work is a queue of pixel tiles over every job of the batch (one job =
-// one render with its own volume, LUT, camera, light, config and size).
-// The job table is the kernel's parameter block, so frame constants are
-// read through the constant cache as in a single-render kernel.  Each
-// 256-thread block pops a tile with one atomic, stages the tile's RGBA LUT
-// (plus the LUT's "clear entry" prefix counts) in shared memory when the
-// job changes, then marches one ray per thread.  Warps cover 8x4-pixel sub-tiles so the rays
-// of a warp are spatially close and their trilinear footprints share cache
-// lines.  Voxels and normals are read from the bricked 16-byte texel
-// records of layout.cu: each sample is 8 vector loads at fixed offsets from
-// one record address.  Paired channels go through the packed FP32x2 pipe,
+// A batch's work is a queue of pixel tiles over every job (one job = one
+// render with its own volume, LUT, camera, light, config and size).  The job
+// table is the kernel's parameter block, so frame constants are read through
+// the constant cache as in a single-render kernel.  Each 256-thread block
+// pops a tile with one atomic, stages the tile's RGBA LUT (plus the LUT's
+// "clear entry" prefix counts) in shared memory when the job changes, then
+// marches one ray per thread; the other kernels stage it once per block, of
+// 256 threads or (single renders of half records) 128.  Warps cover 8x4-pixel
+// sub-tiles so the rays of a warp are spatially close and their trilinear
+// footprints share cache lines.  Voxels and normals are read from the bricked
+// texel records of layout.cu: each sample is 8 vector loads (without normals
+// 2) at fixed offsets from one record address.  Paired channels go through the packed FP32x2 pipe,
 // which rounds each lane exactly like the scalar instruction; an add that
 // consumes a packed product is always a scalar __fadd_rn, so no
 // product/add pair can be fused into one rounding.
@@ -78,8 +80,8 @@ __device__ __forceinline__ float2 half_pair(uint32_t b) {
 // MixedScalar at 40 (it spills) 77 / 139 / 156 / 686, at 48 79 / 119 / 130 /
 // 636, packed Mixed at 48 (spills) 82 / 130 / 135 / 655.  The split kernel at
 // 48: packed (spills) 123 / 291, MixedScalar 113 / 286 (192^2, 256^2 of 512^3).
-// The batch kernels at 48: packed 1498, Mixed 1441; later Mixed 1390,
-// MixedScalar 1440.
+// The batch kernels at 48, two comparisons on two GPUs: packed 1498, Mixed
+// 1441; and Mixed 1390, MixedScalar 1440.
 enum LerpForm { kLerpPacked = 0, kLerpMixed = 1, kLerpMixedScalar = 2 };
 
 template <int LERP>

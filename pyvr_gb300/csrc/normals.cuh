@@ -97,7 +97,7 @@ __device__ __noinline__ float u8_component_f64(float g, float s) {
 __device__ __forceinline__ float u8_component(float g, const U8Norm &n) {
     if (g == 0.0f) return 0.0f;  // +0 / N (numpy's differences of equal values are +0)
     const float qh = __fmul_rn(g, n.r);
-    const float e = fmaf(-qh, n.nh, g);   // g - qh*nh, exact
+    const float e = fmaf(-qh, n.nh, g);   // g - qh*nh, to 2^-46 of g (qh may be an ulp off)
     const float e2 = fmaf(-qh, n.nl, e);  // g - qh*(nh + nl)
     const float corr = __fmul_rn(e2, n.r);
     const float eb = fabsf(qh) * 3.637978807091713e-12f;  // 2^-38 |q|
@@ -154,9 +154,9 @@ __device__ __forceinline__ bool u8_halves(float2 g0, float2 g1, float2 g2, __hal
 // of halves rounded to 24 bits and then to 11 is the one rounded to 11 at
 // once); the sum of squares accumulates in float32 and rounds once.  Its
 // root and the quotients come from approximations and one remainder step
-// each, the remainders exact by FMA (Markstein 1990): RN16 of them equals
-// RN16 of the IEEE results for every half, and for every pair of halves
-// (tests).  False where a sum of squares is 0, infinite or NaN.
+// each, the remainders by FMA (Markstein 1990): RN16 of them equals RN16 of
+// the IEEE results for every half, and for every pair of halves (tests; zeros
+// keep their sign).  False where a sum of squares is 0, infinite or NaN.
 __device__ __forceinline__ float2 half_root(float2 x) {
     const float2 r = make_float2(rsqrt_ftz(x.x), rsqrt_ftz(x.y));
     const float2 s = __fmul2_rn(x, r);
